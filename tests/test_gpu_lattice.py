@@ -41,3 +41,45 @@ def test_lattice_rejects_bad_input(ctx):
         pcf.binom_vanilla_eur(100, 100, .05, .3, 1.0, 0, "put", ctx=ctx)
     with pytest.raises(ValueError):
         pcf.binom_vanilla_amer(100, 100, .05, .3, 1.0, 3_000_000, "put", ctx=ctx)
+
+
+@pytest.mark.parametrize("american", [False, True])
+@pytest.mark.parametrize("N", [8, 9, 23, 24, 25, 31, 33, 191, 192, 193, 3647, 3648])
+def test_lattice_strip_edges_bit_exact(orc, ctx, N, american):
+    """Around the strips' edges: 8 levels between exchanges, 24 columns a warp,
+    24 columns a block up to 152 blocks, then 48. Both are the same FP64
+    operations in the same order, so the prices are equal."""
+    import parcompfin_gb300 as pcf
+    fn = pcf.binom_vanilla_amer if american else pcf.binom_vanilla_eur
+    ref = orc.ref_binom_vanilla_amer if american else orc.ref_binom_vanilla_eur
+    for pf in (1, -1):
+        for args in CASES[:2 if N < 1000 else 1]:
+            assert fn(*args, N, pf, ctx=ctx) == ref(*args, N, float(pf)), (args, N, pf, american)
+
+
+@pytest.mark.parametrize("N", [7296, 10944, 14592])
+def test_lattice_strip_widths_bit_exact(orc, ctx, N):
+    """The first N of 72 and 96 columns a block, and of two blocks an SM."""
+    import parcompfin_gb300 as pcf
+    for american in (True, False):
+        fn = pcf.binom_vanilla_amer if american else pcf.binom_vanilla_eur
+        ref = orc.ref_binom_vanilla_amer if american else orc.ref_binom_vanilla_eur
+        assert fn(100, 110, .02, .75, 1.0, N, -1, ctx=ctx) == ref(100, 110, .02, .75, 1.0, N, -1.0)
+
+
+@pytest.mark.parametrize("american", [False, True])
+@pytest.mark.parametrize("args", [
+    (100, 1e300, .05, .2, 1.0, 300, 1),    # no terminal payoff: the price is 0
+    (1e-280, 2e-280, .05, .2, 1.0, 60, 1),  # a price below 2^-700
+    (100, 100, .05, .2, 1.0, 1, -1),
+    (100, 100, 1.5, .2, 1.0, 1, -1),       # R = e^1.5: beyond the fast division's range
+    (100, 100, -.2, .3, 2.0, 50, -1),      # R < 1
+    (100, 120, .9, .05, 1.0, 2, -1),       # p > 1: negative weights
+])
+def test_lattice_division_range_bit_exact(orc, ctx, args, american):
+    """Prices and parameters outside the three-operation division's range take
+    the IEEE division: the reference's value in every case."""
+    import parcompfin_gb300 as pcf
+    fn = pcf.binom_vanilla_amer if american else pcf.binom_vanilla_eur
+    ref = orc.ref_binom_vanilla_amer if american else orc.ref_binom_vanilla_eur
+    assert fn(*args, ctx=ctx) == ref(*args[:6], float(args[6]))
