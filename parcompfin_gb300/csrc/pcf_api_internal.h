@@ -30,7 +30,7 @@ struct pcf_ctx {
   // log((double)n) table for the reference-order binomial sum.
   double* d_logtab = nullptr;  // one allocation: log table, prefix tables, ties
   int logtab_n = 0;
-  size_t binom_off[4] = {0, 0, 0, 0};  // offsets of prefix sums, tie offsets, ties, stirlerr
+  size_t binom_off[5] = {};  // offsets of prefix sums, tie offsets, ties, stirlerr, 2^(-j/256)
   // Serving slots of pcf_serve_trace, kept between calls (pcf_server.cpp).
   void* serve = nullptr;
   // Upper bound on device bytes this context may hold (0 = unlimited).

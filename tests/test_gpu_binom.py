@@ -160,3 +160,75 @@ def test_edge_cases(orc, ctx):
         binom_embar(100, 100, .05, .2, 1, 2_000_000, 1, ctx=ctx)
     with pytest.raises(ValueError, match="Unknown payoff"):
         binom_embar(100, 100, .05, .2, 1, 100, "straddle", ctx=ctx)
+
+
+def test_reference_mode_small_and_edge_n_vs_oracle(orc, ctx):
+    """Every N up to 70 (the accumulator's low binades, whose ties are dense)
+    and N around multiples of the 256-term blocks and the 32 serial steps of
+    the accumulator's walk, one batch. A term is the reference's up to the
+    rounding of its two powers and its exponential (2^-57 against one ulp) and
+    all terms are positive, so 1e-13 leaves a factor of 100."""
+    from parcompfin_gb300 import binom_embar_batch
+    rng = random.Random(3)
+    cs = [(100.0, rng.uniform(80, 120), rng.uniform(.01, .06), rng.uniform(.1, .5),
+           rng.uniform(.25, 2.0), N, pf)
+          for N in list(range(1, 71)) + [255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 2049]
+          for pf in (1, -1)]
+    for c, v in zip(cs, binom_embar_batch(cs, ctx=ctx)):
+        ref = orc.ref_binom_embar(*c[:6], float(c[6]))
+        assert abs(v - ref) <= 1e-13 * abs(ref) + 1e-300, (c, v, ref)
+
+
+def test_reference_mode_wide_powers_vs_oracle(orc, ctx):
+    """A contract whose powers span almost the whole FP64 range takes the FP64
+    pow and exp; one just below the switch the fixed-point ones. Both agree
+    with the reference's sum, alone and in one batch."""
+    from parcompfin_gb300 import binom_embar, binom_embar_batch
+    N, T = 2000, 4.0
+    cs = []
+    for span in (690.0 - 20.0, 702.0):  # log u times N
+        sig = (span / N) * math.sqrt(N / T)
+        for _ in range(20):  # log u depends on the drift too: settle it
+            lat = (C.c_double * 5)()
+            orc.ref_lattice(.03, sig, T, N, lat)
+            sig *= (span / N) / math.log(lat[0])
+        for pf in (1, -1):
+            cs.append((1.0, 2.0, .03, sig, T, N, pf))
+    got = binom_embar_batch(cs, ctx=ctx)
+    for c, v in zip(cs, got):
+        ref = orc.ref_binom_embar(*c[:6], float(c[6]))
+        assert rel(v, ref) < REF_TOL, (c, v, ref)
+        assert binom_embar(*c, ctx=ctx) == v
+
+
+def _exact_binom(orc, S0, E, r, sig, T, N, pf):
+    """The sum over the lattice's FP64 u, d, p in 60-digit decimals: weights
+    and share prices by their ratios from k = 0."""
+    from decimal import Decimal, getcontext
+    getcontext().prec = 60
+    getcontext().Emin, getcontext().Emax = -10**8, 10**8
+    lat = (C.c_double * 5)()
+    orc.ref_lattice(r, sig, T, N, lat)
+    u, d, p = (Decimal(lat[k]) for k in range(3))
+    q = 1 - p
+    w, S, odds, step = q ** N, Decimal(S0) * d ** N, p / q, u / d
+    total = Decimal(0)
+    for k in range(N + 1):
+        pay = pf * (S - Decimal(E))
+        if pay > 0:
+            total += w * pay
+        w = w * (N - k) / (k + 1) * odds
+        S *= step
+    return math.exp(-r * T) * float(total)
+
+
+@pytest.mark.parametrize("N", [1, 2, 15, 16, 17, 35, 36, 81, 100, 501, 502, 1001, 30_000, 200_000])
+def test_accurate_mode_matches_exact_decimals(orc, ctx, N):
+    """Around the boundaries of the weights' series, at p away from 1/2 too."""
+    from parcompfin_gb300 import binom_embar
+    for r, sig, T, pf in ((.03, .3, 1.5, 1), (.25, .2, 2.0, -1)):
+        if N >= 30_000 and pf < 0:
+            continue
+        ref = _exact_binom(orc, 100.0, 105.0, r, sig, T, N, pf)
+        v = binom_embar(100.0, 105.0, r, sig, T, N, pf, mode="accurate", ctx=ctx)
+        assert abs(v - ref) <= EXACT_TOL * abs(ref), (N, r, v, ref)
