@@ -31,7 +31,8 @@
 //             dates ahead. Each thread updates the exercise decision of its
 //             paths at date m and, in the same pass, adds date m-1's
 //             regression sums in FP32, four consecutive paths per 16-byte
-//             shared-memory load. A warp reduce-scatter leaves the
+//             shared-memory load. Its paths' cash flows and moneyness stay in
+//             its registers. A warp reduce-scatter leaves the
 //             warp's eight sums in eight lanes; after one block barrier a
 //             single warp adds the warp partials and then all CTAs' partials
 //             in double-float, in a fixed order (every CTA gets the same
@@ -41,10 +42,10 @@
 //             averaged over antithetic pairs and reduced with the
 //             deterministic last-block finaliser (cooperative launch) or
 //             through distributed shared memory (cluster launch).
-// Per-path state stays in shared memory for the whole sweep: the cash flow
+// Per-path state stays on the SM for the whole sweep: in registers the cash flow
 // discounted to time 0 (a date's regression target is that times the date's
-// growth factor, which multiplies the date's three y sums once) and the
-// exercise date (8 bits where M <= 255). The
+// growth factor, which multiplies the date's three y sums once), in shared
+// memory the exercise date (8 bits where M <= 255). The
 // regression basis is {1, u, u^2} with u = pf (S - E)/E: the reference's S - E
 // rescaled (and negated for a put), the same fitted values in exact
 // arithmetic. Only paths in the money enter a regression or exercise, so the
@@ -207,16 +208,45 @@ __device__ __forceinline__ void issue_row(const LsmParams& P, int r, long long p
 // has x = 0, so the terms in x add exact zeros without a select; only the
 // count and the y sum test it.
 __device__ __forceinline__ void reg_accumulate(float x, float cfd, float (&acc)[kRegSums]) {
-  const bool itm = x > 0.f;
   const float x2 = x * x;
-  acc[0] += itm ? 1.f : 0.f;
+  // Predicated additions: the compiler's selects cost an instruction more each.
+  asm("{\n\t.reg .pred itm;\n\t"
+      "setp.gt.f32 itm, %2, 0f00000000;\n\t"
+      "@itm add.f32 %0, %0, 0f3F800000;\n\t"
+      "@itm add.f32 %1, %1, %3;\n\t}"
+      : "+f"(acc[0]), "+f"(acc[5])
+      : "f"(x), "f"(cfd));
   acc[1] += x;
   acc[2] += x2;
   acc[3] = fmaf(x2, x, acc[3]);
   acc[4] = fmaf(x2, x2, acc[4]);
-  acc[5] += itm ? cfd : 0.f;
   acc[6] = fmaf(cfd, x, acc[6]);
   acc[7] = fmaf(cfd, x2, acc[7]);
+}
+
+// cfd = v and the exercise date m at shared address `at` + OFF, where x > 0 and
+// ex > cont: one predicate, no branch.
+template <typename TauT, int OFF>
+__device__ __forceinline__ void exercise_if(float x, float ex, float cont, float dm, float& cfd,
+                                            uint32_t at, uint32_t m) {
+  if (sizeof(TauT) == 1)
+    asm volatile("{\n\t.reg .pred go;\n\t"
+                 "setp.gt.f32 go, %1, 0f00000000;\n\t"
+                 "setp.gt.and.f32 go, %2, %3, go;\n\t"
+                 "@go mul.rn.f32 %0, %2, %4;\n\t"
+                 "@go st.shared.u8 [%5+%7], %6;\n\t}"
+                 : "+f"(cfd)
+                 : "f"(x), "f"(ex), "f"(cont), "f"(dm), "r"(at), "r"(m), "n"(OFF)
+                 : "memory");
+  else
+    asm volatile("{\n\t.reg .pred go;\n\t.reg .u16 h;\n\tcvt.u16.u32 h, %6;\n\t"
+                 "setp.gt.f32 go, %1, 0f00000000;\n\t"
+                 "setp.gt.and.f32 go, %2, %3, go;\n\t"
+                 "@go mul.rn.f32 %0, %2, %4;\n\t"
+                 "@go st.shared.u16 [%5+%7], h;\n\t}"
+                 : "+f"(cfd)
+                 : "f"(x), "f"(ex), "f"(cont), "f"(dm), "r"(at), "r"(m), "n"(OFF)
+                 : "memory");
 }
 
 // Reduce-scatter of eight FP32 sums over a warp: each step sends half of the
@@ -443,48 +473,78 @@ __device__ __forceinline__ void regress_date(const LsmParams& P, LsmShared<NW>& 
   }
 }
 
-// Antithetic pair p over the contract's M dates (path p takes +z, path p + H
-// takes -z, as pathsfinder pairs them): writes the positive part of the
-// signed moneyness, x = max(u, 0) with u = pf (S/E - 1), of both paths to the
-// path matrix, one row per date, and returns x at date M of the plus and the
-// minus path. Only x enters the sweep: a path is in the money where x > 0,
-// and its payoff is E x. Date m0 + l + 1 takes
-// lane l of Philox block m0 / 4: whole blocks first, without per-date checks,
-// then the last 1..3 dates.
-__device__ __forceinline__ float2 forward_pair(const LsmParams& P, const RngKey& key,
-                                               long long p) {
+// Antithetic pairs p and p + 1 (p even; the second only if `two`) over the
+// contract's M dates: path p takes +z, path p + H takes -z, as pathsfinder
+// pairs them. Writes the positive part of the signed moneyness, x = max(u, 0)
+// with u = pf (S/E - 1), of the plus and the minus paths to the path matrix,
+// one row per date (0 in the column of a second pair that is not there). Only x
+// enters the sweep: a path is in the money where x > 0, and its payoff is E x.
+// Date m0 + l + 1 takes lane l of Philox block m0 / 4: whole blocks first,
+// without per-date checks, then the last 1..3 dates.
+// Two pairs side by side in packed FP32x2 steps, each lane rounded as the scalar
+// operation, and one 8-byte store for both: a wave of the 64-put batch spends
+// 165 thousand cycles on the pass against 198 with one pair a thread (13.7
+// instructions a path and date; bound by issue, and by HBM's writes next).
+__device__ __forceinline__ void forward_pairs(const LsmParams& P, const RngKey& key, long long p,
+                                              bool two) {
   // The parameters in registers: the stores below go through generic
   // pointers, which the compiler cannot tell apart from P.
   const long long Hp = P.Hp;
   const size_t stride = (size_t)2 * Hp;  // floats per row
-  const float b2 = P.b2, nb2 = -P.b2, a2 = P.a2, pf = P.pf;
+  const float2 b2 = make_float2(P.b2, P.b2), nb2 = make_float2(-P.b2, -P.b2);
+  const float2 a2 = make_float2(P.a2, P.a2);
+  const float2 pf = make_float2(P.pf, P.pf), npf = make_float2(-P.pf, -P.pf);
   const int M = P.M;
-  float Lp = P.l2SE, Lm = P.l2SE, Up = 0.f, Um = 0.f;  // log2(S/E)
-  float* row = P.paths + p;
-  auto step = [&](float z) {
-    Lp += fmaf(b2, z, a2);
-    Lm += fmaf(nb2, z, a2);
-    Up = fmaxf(fmaf(pf, ex2_approx(Lp), -pf), 0.f);  // max(pf (S/E - 1), 0)
-    Um = fmaxf(fmaf(pf, ex2_approx(Lm), -pf), 0.f);
-    row[0] = Up;
-    row[Hp] = Um;
-    row += stride;
+  float2 Lp = make_float2(P.l2SE, P.l2SE), Lm = Lp;  // log2(S/E)
+  float* plus = P.paths + p;
+  float* minus = plus + Hp;
+  auto moneyness = [&](float2 L) {
+    const float2 u = __ffma2_rn(pf, make_float2(ex2_approx(L.x), ex2_approx(L.y)), npf);
+    return make_float2(fmaxf(u.x, 0.f), two ? fmaxf(u.y, 0.f) : 0.f);
+  };
+  auto step = [&](float2 z) {
+    Lp = __fadd2_rn(Lp, __ffma2_rn(b2, z, a2));
+    Lm = __fadd2_rn(Lm, __ffma2_rn(nb2, z, a2));
+    *reinterpret_cast<float2*>(plus) = moneyness(Lp);
+    *reinterpret_cast<float2*>(minus) = moneyness(Lm);
+    plus += stride;
+    minus += stride;
   };
   const int Mfull = M & ~3;
   for (int m0 = 0; m0 < Mfull; m0 += 4) {
-    const float4 z4 = normals4(draw_words(key, (uint64_t)p, (uint32_t)(m0 >> 2)));
-    step(z4.x);
-    step(z4.y);
-    step(z4.z);
-    step(z4.w);
+    float2 z[4];
+    normals4_pair(draw_words(key, (uint64_t)p, (uint32_t)(m0 >> 2)),
+                  draw_words(key, (uint64_t)(p + 1), (uint32_t)(m0 >> 2)), z);
+    step(z[0]);
+    step(z[1]);
+    step(z[2]);
+    step(z[3]);
   }
   if (Mfull < M) {
-    const float4 z4 = normals4(draw_words(key, (uint64_t)p, (uint32_t)(Mfull >> 2)));
-    step(z4.x);
-    if (Mfull + 1 < M) step(z4.y);
-    if (Mfull + 2 < M) step(z4.z);
+    float2 z[4];
+    normals4_pair(draw_words(key, (uint64_t)p, (uint32_t)(Mfull >> 2)),
+                  draw_words(key, (uint64_t)(p + 1), (uint32_t)(Mfull >> 2)), z);
+    step(z[0]);
+    if (Mfull + 1 < M) step(z[1]);
+    if (Mfull + 2 < M) step(z[2]);
   }
-  return make_float2(Up, Um);
+}
+
+// The forward pass of a block's pairs [p0, p0 + nb), padded with columns of 0
+// (out of the money: they never exercise and add nothing) to a multiple of
+// four, the width of the bulk copies and of the sweep's steps.
+template <int BS>
+__device__ __forceinline__ void forward_block(const LsmParams& P, const RngKey& key, long long p0,
+                                              long long nb) {
+  for (long long i = 2 * threadIdx.x; i < nb; i += 2 * BS)
+    forward_pairs(P, key, p0 + i, i + 1 < nb);
+  const long long nbr = (nb + 3) & ~3LL;
+  const size_t stride = (size_t)2 * P.Hp;
+  for (long long i = ((nb + 1) & ~1LL) + threadIdx.x; i < nbr; i += BS)
+    for (int m = 0; m < P.M; ++m) {
+      P.paths[(size_t)m * stride + p0 + i] = 0.f;
+      P.paths[(size_t)m * stride + P.Hp + p0 + i] = 0.f;
+    }
 }
 
 // The control-variate sample of one path with exercise date tau, cash flow
@@ -512,7 +572,15 @@ __device__ __forceinline__ float cv_sample(const LsmParams& P, const float* dt, 
 // cooperative block that gave up leaves after its in-flight copies landed; a
 // cluster CTA records the failure and keeps taking part in every exchange and
 // cluster barrier (a hardware barrier has no timeout), so no CTA leaves early.
-template <int MODE, typename TauT, int BS>
+//
+// A thread keeps its J groups of four consecutive pairs for the whole sweep:
+// their cash flows and the moneyness at the date being decided stay in
+// registers (16 J values), so that a pass loads one 16-byte slice of the next
+// date per four paths from shared memory and stores nothing but exercise dates.
+// With both in shared memory the pass moved five times as much there. The pass
+// is bound by issue; with registers and predicated updates it takes 1850 cycles
+// against 2700 (64-put batch), and the batch 552 us against 589.
+template <int MODE, typename TauT, int BS, int J>
 __device__ void lsm_body(const LsmParams& P, int b, int rank) {
   constexpr bool CLUSTER = MODE == kCluster;  // one cluster per contract
   constexpr bool DSMEM = MODE != kCoop;       // CTAs exchange through cluster shared memory
@@ -544,32 +612,39 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
 
   // ---- forward: generate and store paths ----
   const RngKey key{P.seed_lo, P.seed_hi, P.stream, TAG_AMER};
-  const float EdM = P.E * P.dtab[M];  // payoff at T = E max(u, 0), discounted
-  const size_t stride = (size_t)2 * P.Hp;  // floats per row
-#pragma unroll 2
-  for (int i = threadIdx.x; i < nb; i += BS) {
-    const float2 uM = forward_pair(P, key, p0 + i);
-    S.cf[i] = fmaxf(uM.x, 0.f) * EdM;
-    S.cf[PB + i] = fmaxf(uM.y, 0.f) * EdM;
-    S.tau[i] = (TauT)M;
-    S.tau[PB + i] = (TauT)M;
-  }
-  // Columns [nb, nbr) pad the last block's bulk copies to 16 bytes: u = 0 and
-  // cf = 0 there, so the four-path steps below see paths out of the money
-  // that never exercise and add nothing.
-  for (int i = nb + threadIdx.x; i < nbr; i += BS) {
-    for (int m = 0; m < M; ++m) {
-      P.paths[(size_t)m * stride + p0 + i] = 0.f;
-      P.paths[(size_t)m * stride + P.Hp + p0 + i] = 0.f;
-    }
-    S.cf[i] = 0.f;
-    S.cf[PB + i] = 0.f;
-  }
+  forward_block<BS>(P, key, p0, nb);
   // The bulk copies below read what this block's threads just stored; the
   // cluster barrier also publishes the exchange mbarriers to the peers.
   fence_proxy_async_global();
   if (DSMEM) cg::this_cluster().sync();
   else __syncthreads();
+
+  // This thread's paths: pairs 4 (tid + k BS) .. + 3, k < J, the plus paths then
+  // the minus paths. The cash flow at T is the payoff E x, discounted to 0.
+  float cf[J][8], u[J][8];
+  {
+    const float EdM = P.E * P.dtab[M];
+    const float* last = P.paths + (size_t)(M - 1) * 2 * P.Hp + p0;
+#pragma unroll
+    for (int k = 0; k < J; ++k) {
+      const int j = threadIdx.x + k * BS;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j < nq) {
+          x = *reinterpret_cast<const float4*>(last + h * P.Hp + 4 * j);
+#pragma unroll
+          for (int l = 0; l < 4; ++l) S.tau[h * PB + 4 * j + l] = (TauT)M;
+        }
+        cf[k][4 * h] = x.x * EdM;
+        cf[k][4 * h + 1] = x.y * EdM;
+        cf[k][4 * h + 2] = x.z * EdM;
+        cf[k][4 * h + 3] = x.w * EdM;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) u[k][4 * h + l] = 0.f;
+      }
+    }
+  }
 
   // Buffer schedule: date d's slice sits in buf[(M - 1 - d) & 1]. Thread 32
   // issues every copy; every thread waits on the copy it is about to read.
@@ -607,43 +682,50 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
     __syncthreads();
   };
 
+  const uint32_t tau_at = smem_u32(S.tau + 4 * threadIdx.x);  // the thread's first exercise date
+  // Loads the slice's values of group k into u and adds the date's sums.
+  auto gather = [&](const float* sl, int k, float (&acc)[kRegSums]) {
+    const int j = threadIdx.x + k * BS;
+    if (J > 1 && j >= nq) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (J > 1 || j < nq) x = ld4(sl + h * PB + 4 * j);
+      u[k][4 * h] = x.x;
+      u[k][4 * h + 1] = x.y;
+      u[k][4 * h + 2] = x.z;
+      u[k][4 * h + 3] = x.w;
+#pragma unroll
+      for (int l = 0; l < 4; ++l) reg_accumulate(u[k][4 * h + l], cf[k][4 * h + l], acc);
+    }
+  };
+
   // Sums for date M-1 (the only date without a preceding update pass).
   {
     wait_copy(0);
     float acc[kRegSums];
 #pragma unroll
     for (int q = 0; q < kRegSums; ++q) acc[q] = 0.f;
-    const float* sl = S.slice(0);
-    for (int j = threadIdx.x; j < nq; j += BS) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int s = h * PB + 4 * j;
-        const float4 u = ld4(sl + s), c = ld4(S.cf + s);
-        reg_accumulate(u.x, c.x, acc);
-        reg_accumulate(u.y, c.y, acc);
-        reg_accumulate(u.z, c.z, acc);
-        reg_accumulate(u.w, c.w, acc);
-      }
-    }
+    for (int k = 0; k < J; ++k) gather(S.slice(0), k, acc);
     regress(acc, M - 1, -1, 0);
   }
 
   // Date m: update with date m's coefficients, fused with the sums of date m-1.
   bool failed = !DSMEM && X.fail;
   for (int m = M - 1; m >= 1 && !failed; --m) {
-    const int k = (M - 1 - m) & 1;
+    const int kb = (M - 1 - m) & 1;
     const bool has_next = m > 1;
-    if (has_next) wait_copy(k ^ 1);
+    if (has_next) wait_copy(kb ^ 1);
     const int mode = X.mode;
     const float c0 = X.coef[0], c1 = X.coef[1], c2 = X.coef[2];
     const float dm = S.dt[m], em = S.edt[m];
-    const float* cur = S.slice(k);
-    const float* nxt = S.slice(k ^ 1);
+    const float* nxt = S.slice(kb ^ 1);
     float acc[kRegSums];
 #pragma unroll
     for (int q = 0; q < kRegSums; ++q) acc[q] = 0.f;
     const float E = P.E, nK = P.nK;
-    // One pass over the block's paths, compiled once per case (the date's
+    // One pass over the thread's paths, compiled once per case (the date's
     // mode MD, the reference's exercise rule RX, a following date NX), so
     // the loop carries no per-path test of them.
     auto sweep = [&](auto md_c, auto rx_c, auto nx_c) {
@@ -653,46 +735,32 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
       // Exercise decision at date m (src/mc_amer.cpp:73-106) for one path:
       // exercise where the path is in the money and the payoff beats the
       // continuation value; the cash flow becomes the payoff discounted to 0.
-      auto decide = [&](float u, float& cfd, int s) {  // u: the stored max(u, 0)
-        float cont, ex = u * E;  // the payoff E max(u, 0)
+      auto decide = [&](float x, float& cfd, uint32_t at, auto off) {  // x: the stored max(u, 0)
+        float cont, ex = x * E;  // the payoff E max(u, 0)
         if (MD == 1) {
           cont = cfd * em;
         } else {
-          cont = fmaf(fmaf(c2, u, c1), u, c0);
+          cont = fmaf(fmaf(c2, x, c1), x, c0);
           // src/mc_amer.cpp:100: the reference exercises at payoff(S - E, E),
           // max(pf (S - 2E), 0) = max(E u - pf E, 0).
-          if (RX) ex = fmaxf(fmaf(E, u, nK), 0.f);
+          if (RX) ex = fmaxf(fmaf(E, x, nK), 0.f);
         }
-        if (u > 0.f && ex > cont) {
-          cfd = ex * dm;
-          S.tau[s] = (TauT)m;
-        }
+        exercise_if<TauT, decltype(off)::value * (int)sizeof(TauT)>(x, ex, cont, dm, cfd, at,
+                                                                    (uint32_t)m);
       };
-#pragma unroll 2
-      for (int j = threadIdx.x; j < nq; j += BS) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int s = h * PB + 4 * j;
-          float4 c = ld4(S.cf + s);
-          // Date m-1's slice is not written by this pass: load it before the
-          // exercise update's stores, so its latency overlaps the update.
-          const float4 un = NX ? ld4(nxt + s) : make_float4(0.f, 0.f, 0.f, 0.f);
-          if (MD != 0) {
-            const float4 u = ld4(cur + s);
-            decide(u.x, c.x, s);
-            decide(u.y, c.y, s + 1);
-            decide(u.z, c.z, s + 2);
-            decide(u.w, c.w, s + 3);
-            st4(S.cf + s, c);
-          }
-          if (NX) {
-            const float4 u = un;
-            reg_accumulate(u.x, c.x, acc);
-            reg_accumulate(u.y, c.y, acc);
-            reg_accumulate(u.z, c.z, acc);
-            reg_accumulate(u.w, c.w, acc);
+      for (int k = 0; k < J; ++k) {
+        if (MD != 0) {  // an idle thread's paths have x = 0: they never exercise
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t at = tau_at + (uint32_t)((h * PB + 4 * k * BS) * sizeof(TauT));
+            decide(u[k][4 * h], cf[k][4 * h], at, std::integral_constant<int, 0>{});
+            decide(u[k][4 * h + 1], cf[k][4 * h + 1], at, std::integral_constant<int, 1>{});
+            decide(u[k][4 * h + 2], cf[k][4 * h + 2], at, std::integral_constant<int, 2>{});
+            decide(u[k][4 * h + 3], cf[k][4 * h + 3], at, std::integral_constant<int, 3>{});
           }
         }
+        if (NX) gather(nxt, k, acc);
       }
     };
     using Md0 = std::integral_constant<int, 0>;
@@ -712,9 +780,20 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
       else if (mode == 2) sweep(Md2{}, No{}, No{});
     }
     if (!has_next) break;
-    regress(acc, m - 1, m - 2 >= 1 ? m - 3 : -1, k);
+    regress(acc, m - 1, m - 2 >= 1 ? m - 3 : -1, kb);
     failed = !DSMEM && X.fail;
   }
+  if (!failed)  // the final sums go over the pairs in another order
+#pragma unroll
+    for (int k = 0; k < J; ++k) {
+      const int j = threadIdx.x + k * BS;
+      if (j < nq) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          st4(S.cf + h * PB + 4 * j, make_float4(cf[k][4 * h], cf[k][4 * h + 1], cf[k][4 * h + 2],
+                                                 cf[k][4 * h + 3]));
+      }
+    }
   __syncthreads();
   if (failed) {
     // Let any bulk copy this block issued land before the block exits.
@@ -774,13 +853,16 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
   }
 }
 
+// J: groups of four pairs a thread holds (1, 2 or 4), as the slice asks.
+template <int J>
 __global__ void __launch_bounds__(kLsmBlock, 1) lsm_kernel(LsmParams P) {
-  lsm_body<kCoop, unsigned short, kLsmBlock>(P, blockIdx.x, 0);
+  lsm_body<kCoop, unsigned short, kLsmBlock, J>(P, blockIdx.x, 0);
 }
 
 // One large contract on a cooperative grid of clusters (P.cluster CTAs each):
 // per date the CTAs of a cluster exchange through distributed shared memory,
 // and only the clusters' leaders meet in global memory.
+template <int J>
 __global__ void __launch_bounds__(kLsmBlock, 1) lsm_coop_cluster_kernel(LsmParams P) {
   // The exchange addresses P.cluster peers: a launch without that cluster
   // shape stops here with an error instead of addressing absent CTAs.
@@ -788,8 +870,8 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_coop_cluster_kernel(LsmParam
     if (threadIdx.x == 0) atomicExch(P.err, 4);
     return;
   }
-  lsm_body<kCoopCluster, unsigned short, kLsmBlock>(P, blockIdx.x,
-                                                    (int)cg::this_cluster().block_rank());
+  lsm_body<kCoopCluster, unsigned short, kLsmBlock, J>(P, blockIdx.x,
+                                                       (int)cg::this_cluster().block_rank());
 }
 
 // Streaming sweep for a contract whose per-block slice does not fit in
@@ -818,25 +900,20 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_stream_kernel(LsmParams P) {
   }
   if (threadIdx.x == 0) X.fail = 0;
 
-  // ---- forward: the whole-path loop of lsm_body ----
+  // ---- forward: as lsm_body ----
   const RngKey key{P.seed_lo, P.seed_hi, P.stream, TAG_AMER};
   const float EdM = P.E * P.dtab[M];
   const size_t stride = (size_t)2 * Hp;
-  for (long long i = threadIdx.x; i < nb; i += BS) {
-    const long long p = p0 + i;
-    const float2 uM = forward_pair(P, key, p);
-    P.gcf[p] = fmaxf(uM.x, 0.f) * EdM;
-    P.gcf[Hp + p] = fmaxf(uM.y, 0.f) * EdM;
-    P.gtau[p] = (unsigned short)M;
-    P.gtau[Hp + p] = (unsigned short)M;
-  }
-  for (long long i = nb + threadIdx.x; i < nbr; i += BS) {  // padding: out of the money
-    for (int m = 0; m < M; ++m) {
-      P.paths[(size_t)m * stride + p0 + i] = 0.f;
-      P.paths[(size_t)m * stride + Hp + p0 + i] = 0.f;
+  forward_block<BS>(P, key, p0, nb);
+  __syncthreads();
+  for (long long i = threadIdx.x; i < nbr; i += BS) {
+    const float* last = P.paths + (size_t)(M - 1) * stride + p0 + i;
+    P.gcf[p0 + i] = last[0] * EdM;
+    P.gcf[Hp + p0 + i] = last[Hp] * EdM;
+    if (i < nb) {
+      P.gtau[p0 + i] = (unsigned short)M;
+      P.gtau[Hp + p0 + i] = (unsigned short)M;
     }
-    P.gcf[p0 + i] = 0.f;
-    P.gcf[Hp + p0 + i] = 0.f;
   }
   __syncthreads();  // every path of the block is read below by another thread
 
@@ -956,8 +1033,8 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_stream_kernel(LsmParams P) {
 // (cluster size = the contracts' common CTA count). Two CTAs per SM: while
 // one runs its per-date exchange and solve, the other's paths keep the SM
 // busy.
-template <typename TauT>
-__global__ void __launch_bounds__(kLsmCBlock, 2)
+template <typename TauT, int J>
+__global__ void __launch_bounds__(kLsmCBlock, J > 2 ? 1 : 2)
     lsm_cluster_kernel(const LsmParams* __restrict__ cs, int C) {
   __shared__ LsmParams sP;  // the contract's parameters, read from shared memory
   const unsigned rank = cg::this_cluster().block_rank();
@@ -971,7 +1048,36 @@ __global__ void __launch_bounds__(kLsmCBlock, 2)
   const int c = (int)(blockIdx.x / CL);
   if (threadIdx.x == 0) sP = cs[c];
   __syncthreads();
-  lsm_body<kCluster, TauT, kLsmCBlock>(sP, (int)rank, (int)rank);
+  lsm_body<kCluster, TauT, kLsmCBlock, J>(sP, (int)rank, (int)rank);
+}
+
+// Groups of four pairs a thread of a 512-thread block holds for a slice of PB
+// pairs: the kernels' J.
+int lsm_groups(int PB) {
+  const int k = (PB / 4 + kLsmBlock - 1) / kLsmBlock;
+  return k <= 1 ? 1 : k <= 2 ? 2 : 4;
+}
+static_assert(kLsmBlock == kLsmCBlock, "lsm_groups serves both");
+typedef void (*LsmKernel)(LsmParams);
+typedef void (*LsmClusterKernel)(const LsmParams*, int);
+LsmKernel lsm_kernel_for(int PB) {
+  const int k = lsm_groups(PB);
+  return k == 1 ? lsm_kernel<1> : k == 2 ? lsm_kernel<2> : lsm_kernel<4>;
+}
+LsmKernel lsm_hybrid_for(int PB) {
+  const int k = lsm_groups(PB);
+  return k == 1 ? lsm_coop_cluster_kernel<1> : k == 2 ? lsm_coop_cluster_kernel<2>
+                                                      : lsm_coop_cluster_kernel<4>;
+}
+LsmClusterKernel lsm_cluster_for(int PB, bool t8) {
+  const int k = lsm_groups(PB);
+  if (t8)
+    return k == 1   ? lsm_cluster_kernel<unsigned char, 1>
+           : k == 2 ? lsm_cluster_kernel<unsigned char, 2>
+                    : lsm_cluster_kernel<unsigned char, 4>;
+  return k == 1   ? lsm_cluster_kernel<unsigned short, 1>
+         : k == 2 ? lsm_cluster_kernel<unsigned short, 2>
+                  : lsm_cluster_kernel<unsigned short, 4>;
 }
 
 // Dynamic shared memory of one block (the carve above).
@@ -1072,16 +1178,17 @@ const LsmLimits& lsm_limits(const pcf_ctx* c) {
     L.status = cuda_status(
         cudaDeviceGetAttribute(&v, cudaDevAttrReservedSharedMemoryPerBlock, c->device), "attr");
   L.reserved = (size_t)v;
-  if (!L.status) L.status = lsm_kernel_setup(lsm_kernel, L.per_block, &L.stat_coop, false);
-  if (!L.status) {
-    size_t stat = 0;
-    L.status = lsm_kernel_setup(lsm_coop_cluster_kernel, L.per_block, &stat, false);
-    L.stat_coop = std::max(L.stat_coop, stat);
+  for (int PB : {kLsmBlock * 4, kLsmBlock * 8, kLsmBlock * 16}) {
+    auto setup = [&](auto kernel, size_t& most, bool cluster) {
+      size_t stat = 0;
+      if (!L.status) L.status = lsm_kernel_setup(kernel, L.per_block, &stat, cluster);
+      most = std::max(most, stat);
+    };
+    setup(lsm_kernel_for(PB), L.stat_coop, false);
+    setup(lsm_hybrid_for(PB), L.stat_coop, false);
+    setup(lsm_cluster_for(PB, true), L.stat8, true);
+    setup(lsm_cluster_for(PB, false), L.stat16, true);
   }
-  if (!L.status)
-    L.status = lsm_kernel_setup(lsm_cluster_kernel<unsigned char>, L.per_block, &L.stat8, true);
-  if (!L.status)
-    L.status = lsm_kernel_setup(lsm_cluster_kernel<unsigned short>, L.per_block, &L.stat16, true);
   if (!L.status) {
     // 16-CTA clusters where the device can co-schedule them at two CTAs per
     // SM with 4096-pair slices; otherwise the portable 8.
@@ -1097,7 +1204,7 @@ const LsmLimits& lsm_limits(const pcf_ctx* c) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int n = 0;
-    L.cl_max = cudaOccupancyMaxActiveClusters(&n, lsm_cluster_kernel<unsigned char>, &cfg) ==
+    L.cl_max = cudaOccupancyMaxActiveClusters(&n, lsm_cluster_for(4096, true), &cfg) ==
                            cudaSuccess &&
                        n > 0
                    ? 16
@@ -1169,7 +1276,8 @@ void hybrid_shape(const LsmLimits& Lm, long long H, int M, int G, size_t smem, i
     q.attrs = qa;
     q.numAttrs = 1;
     int ncl = 0;
-    if (cudaOccupancyMaxActiveClusters(&ncl, lsm_coop_cluster_kernel, &q) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveClusters(&ncl, lsm_hybrid_for((int)((H + G - 1) / G)), &q) !=
+        cudaSuccess) {
       cudaGetLastError();
       continue;
     }
@@ -1210,7 +1318,7 @@ int launch_coop(const LsmParams& P0, int G, int PB, size_t smem, int hcl, int Gh
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 2;
-    if (cudaLaunchKernelEx(&cfg, lsm_coop_cluster_kernel, P) == cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, lsm_hybrid_for(PBh), P) == cudaSuccess) {
       *used_hybrid = true;
       return PCF_OK;
     }
@@ -1220,7 +1328,7 @@ int launch_coop(const LsmParams& P0, int G, int PB, size_t smem, int hcl, int Gh
   P.nblocks = G;
   P.cluster = 0;
   void* args[] = {&P};
-  return cuda_status(cudaLaunchCooperativeKernel((void*)lsm_kernel, dim3(G), dim3(kLsmBlock), args,
+  return cuda_status(cudaLaunchCooperativeKernel((void*)lsm_kernel_for(PB), dim3(G), dim3(kLsmBlock), args,
                                                  smem, s),
                      "lsm cooperative launch");
 }
@@ -1529,8 +1637,7 @@ int lsm_batch_launch_clusters(pcf_ctx* c, LsmBatch* B, cudaStream_t s) {
     cfg.numAttrs = 1;
     const LsmParams* prm = L.d_params;
     const int C = L.C;
-    st = cuda_status(L.t8 ? cudaLaunchKernelEx(&cfg, lsm_cluster_kernel<unsigned char>, prm, C)
-                          : cudaLaunchKernelEx(&cfg, lsm_cluster_kernel<unsigned short>, prm, C),
+    st = cuda_status(cudaLaunchKernelEx(&cfg, lsm_cluster_for(L.PB, L.t8), prm, C),
                      "lsm cluster launch");
     if (st) return st;
     c->launches += 1;
@@ -1608,7 +1715,7 @@ int amer_run(pcf_ctx* ctx, double S0, double E, double r, double sigma, double T
   } else {
     int occ = 0;
     st = cuda_status(
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, lsm_kernel, kLsmBlock, smem),
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, lsm_kernel_for(PB), kLsmBlock, smem),
         "occupancy(lsm)");
     if (st) return st;
     if ((long long)occ * c->sm_count < G)

@@ -119,6 +119,33 @@ __device__ __forceinline__ float4 normals4_x2(uint4 w) {
   return make_float4(c.x, s.x, c.y, s.y);
 }
 
+// normals4 of two Philox blocks side by side: z[l] holds normal l of block a
+// (.x) and of block b (.y), ready for packed steps of the two paths. The same
+// bits as normals4 of each.
+__device__ __forceinline__ void normals4_pair(uint4 a, uint4 b, float2 (&z)[4]) {
+  const float kNeg2Ln2 = -1.38629436112f;
+  auto radius = [&](uint32_t wa, uint32_t wb) {
+    const float2 f = __fadd2_rn(make_float2(__uint_as_float(0x3f800000u | (wa >> 9)),
+                                            __uint_as_float(0x3f800000u | (wb >> 9))),
+                                make_float2(-0.99999994f, -0.99999994f));  // uniform_open
+    const float2 l = __fmul2_rn(make_float2(kNeg2Ln2, kNeg2Ln2),
+                                make_float2(lg2_approx(f.x), lg2_approx(f.y)));
+    return make_float2(sqrt_approx(l.x), sqrt_approx(l.y));
+  };
+  auto angle = [&](uint32_t wa, uint32_t wb) {
+    return __ffma2_rn(make_float2(3.14159265359f, 3.14159265359f),
+                      make_float2(__uint_as_float(0x40000000u | (wa >> 9)),
+                                  __uint_as_float(0x40000000u | (wb >> 9))),
+                      make_float2(-9.42477758f, -9.42477758f));  // bm_angle
+  };
+  const float2 r0 = radius(a.x, b.x), t0 = angle(a.y, b.y);
+  const float2 r1 = radius(a.z, b.z), t1 = angle(a.w, b.w);
+  z[0] = __fmul2_rn(r0, make_float2(cos_approx(t0.x), cos_approx(t0.y)));
+  z[1] = __fmul2_rn(r0, make_float2(sin_approx(t0.x), sin_approx(t0.y)));
+  z[2] = __fmul2_rn(r1, make_float2(cos_approx(t1.x), cos_approx(t1.y)));
+  z[3] = __fmul2_rn(r1, make_float2(sin_approx(t1.x), sin_approx(t1.y)));
+}
+
 __device__ __forceinline__ float lane4(const float4& v, int l) {
   return l == 0 ? v.x : (l == 1 ? v.y : (l == 2 ? v.z : v.w));
 }
