@@ -11,12 +11,12 @@
 //   cooperative  one contract per launch, at most one 512-thread block per
 //                SM (pcf_mc_amer, and batch contracts too large for a
 //                cluster). Blocks exchange their partial sums through global
-//                memory and a bounded group barrier;
+//                memory, each word with its date (bounded waits);
 //   cluster      many contracts per launch, one thread-block cluster per
 //                contract (pcf_plan_*). CTAs write their partial sums into
 //                every peer's shared memory and signal the peer's mbarrier;
 //   cooperative grid of clusters  one large contract: the cluster exchange,
-//                then only the cluster leaders meet in global memory;
+//                then one total per cluster through global memory;
 //   streaming    one contract whose per-block slice exceeds shared memory
 //                (lsm_stream_kernel): per-path state in device memory.
 // Phases:
@@ -28,7 +28,7 @@
 //             [Hp, 2Hp), Hp = H rounded up to 4), coalesced across the warp;
 //   backward  for m = M-1..1 the block's slice of row m-1 (two contiguous
 //             runs) arrives in shared memory by TMA bulk copy, issued two
-//             dates ahead. Each thread updates the exercise decision of its
+//             dates before it is read. Each thread updates the exercise decision of its
 //             paths at date m and, in the same pass, adds date m-1's
 //             regression sums in FP32, four consecutive paths per 16-byte
 //             shared-memory load. Its paths' cash flows and moneyness stay in
@@ -79,7 +79,7 @@ constexpr int kMaxCluster = 16;  // CTAs per contract in a cluster launch
 
 // How the CTAs of one contract exchange their per-date sums.
 enum LsmMode : int {
-  kCoop = 0,         // cooperative grid: global memory and a group barrier
+  kCoop = 0,         // cooperative grid: global memory
   kCluster = 1,      // one thread-block cluster: distributed shared memory
   kCoopCluster = 2,  // cooperative grid of clusters: both, in two levels
 };
@@ -95,17 +95,17 @@ struct LsmParams {
   int nblocks;            // blocks (cooperative) or CTAs of the cluster
   int cluster;            // hybrid launch: CTAs per cluster (nblocks is a multiple)
   uint32_t seed_lo, seed_hi, stream;
-  unsigned wait_limit;       // group-barrier polls before giving up
+  unsigned wait_limit;       // polls for the other blocks' totals before giving up
   unsigned copy_wait_limit;  // mbarrier polls before giving up
-  unsigned barrier_extra;    // test hook: arrivals the cooperative group barrier expects
-                             // beyond the grid (it can then never complete); 0 otherwise
+  unsigned barrier_extra;    // test hook: the cooperative exchange expects a total that no
+                             // block publishes (it can then never complete); 0 otherwise
   float* paths;           // M rows of 2*Hp floats
   const float* dtab;      // exp(-r dt k), k = 0..M, then exp(+r dt k), k = 0..M
-  double* partial;        // 2 x nblocks x kRegSums (cooperative)
+  double* partial;        // cooperative: two slots of (nblocks + 1) x kRegSums 16-byte totals,
+                          // 0 at launch
   double* fpartial;       // nblocks x kMoments (cooperative)
-  unsigned* barrier;
   unsigned* ticket;
-  int* err;               // 1: a barrier wait gave up, 2: a bulk copy wait gave up,
+  int* err;               // 1: a wait on other blocks gave up, 2: a bulk copy wait gave up,
                           // 4: the launch lacked its cluster shape (nothing computed)
   int* singular;          // dates whose normal equations had det <= 0
   double* out;            // kMoments sums
@@ -171,18 +171,25 @@ __device__ __forceinline__ LsmSmem<TauT> carve(unsigned char* base, int PB, int 
   return s;
 }
 
+// The totals of nblocks blocks (and one word more, of the test hook) fit in the
+// place of a block's 2 PB cash flows.
+__host__ __device__ __forceinline__ bool exchange_fits(int PB, int nblocks) {
+  return (size_t)2 * PB * sizeof(float) >= ((size_t)nblocks + 1) * kRegSums * sizeof(DF);
+}
+// Shared memory a cooperative block needs for them otherwise.
+__host__ __device__ __forceinline__ size_t exchange_bytes(int PB, int nblocks) {
+  return exchange_fits(PB, nblocks) ? 0 : ((size_t)nblocks + 1) * kRegSums * sizeof(DF);
+}
+
 // Static shared memory of one block of NW warps: the exchange of regression
 // sums.
 template <int NW>
 struct LsmShared {
   float wpart[NW][kRegSums];                     // per-warp FP32 sums
   alignas(16) DF xin[2][kMaxCluster][kRegSums];  // cluster: every CTA's totals, by date parity
-  alignas(16) DF ctot[kRegSums];                 // this CTA's totals
   uint64_t xbar[2];                              // cluster: bytes of the CTAs' totals
-  DF tdf[kRegSums];                              // the contract's sums, scaled
-  DF cof[8];                                     // adjugate of the normal matrix
-  float coef[3];
-  int mode;  // 0 skip the date, 1 few in-the-money paths, 2 regression
+  alignas(16) float coef[4];  // c0, c1, c2 and the mode's bits: 0 skip the date, 1 few
+                              // in-the-money paths, 2 regression
   int fail;  // a wait gave up
   DF sh[NW * kMoments];
   DF fin[kMoments];
@@ -275,132 +282,138 @@ __device__ __forceinline__ float warp_scatter8(const float (&a)[kRegSums]) {
   return v;
 }
 
-// Cooperative launch: arrival at the group barrier by one thread, after the
-// block's partials were stored and fenced. `counter` only grows: arrival
-// number a (0-based) waits until the count reaches (a/G + 1)*G. Bounded: after
-// `limit` polls (or once another block reported a failure) it raises *err and
-// returns false.
-__device__ __forceinline__ bool group_arrive_wait(unsigned* counter, unsigned G, int* err,
-                                                  unsigned limit) {
-  const unsigned a = atomicAdd(counter, 1u);
-  const unsigned target = (a / G + 1u) * G;
-  for (unsigned polls = 0;; ++polls) {
-    const unsigned c = *((volatile unsigned*)counter);
-    if ((int)(c - target) >= 0) break;
-    if (*((volatile int*)err) != 0 || polls > limit) {
-      atomicExch(err, 1);
-      return false;
-    }
-    __nanosleep(32);
-  }
-  __threadfence();
-  return true;
+// Exchange of totals through global memory (cooperative launches): a total
+// travels as two 8-byte words {FP32 value, date}, each written and read
+// atomically, so the date says that the word has arrived: no fence, no counter
+// and no second round trip for the data. The words of a launch start at 0 (no
+// date). Two slots by the date's parity are enough: a block writes date d after
+// it has every block's date d + 1, which each sent after it had read all of
+// date d + 2. A fence, an atomic counter, its polls and then the loads took 6500
+// to 7900 cycles a date; this takes 2000 to 2600, the latency of a store and a
+// load across the L2 (10^5 paths, 200 dates: 1.10 -> 0.59 ms; 2^20 paths, 50
+// dates: 0.33 -> 0.23 ms).
+__device__ __forceinline__ void publish_total(void* slot, int item, DF v, int d) {
+  const unsigned long long hi = (unsigned long long)__float_as_uint(v.hi) |
+                                ((unsigned long long)(unsigned)d << 32);
+  const unsigned long long lo = (unsigned long long)__float_as_uint(v.lo) |
+                                ((unsigned long long)(unsigned)d << 32);
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"((char*)slot + 16 * (size_t)item),
+               "l"(hi), "l"(lo)
+               : "memory");
 }
 
-// Date d's regression, run by warp 0 between the two block barriers: the
-// block's total of each sum, the exchange of block totals, the contract's
-// sums in FP64 and the solve. Leaves the mode and coefficients in X.
-template <int MODE, int NW>
-__device__ __forceinline__ void regress_date(const LsmParams& P, LsmShared<NW>& X, int d, int b,
-                                             int rank, uint32_t& xph, uint32_t& xcount,
-                                             float growth) {
-  const int lane = threadIdx.x & 31;
-  const int q = lane & 7;
-  // Block total of sum q: lane groups l>>3 = 0..3 each add four warps' sums,
-  // then two shuffle steps combine the groups. Lanes 0..7 hold the totals.
+// All threads of the block: waits for date d's `items` totals and copies them
+// to shared memory. Bounded: after `limit` polls (or once another block reported
+// a failure) it raises *err and returns false in the threads that gave up.
+template <int BS>
+__device__ __forceinline__ bool gather_totals(const void* slot, int items, int d, DF* to, int* err,
+                                              unsigned limit) {
+  constexpr int kBatch = 3;  // loads in flight a thread: 192 blocks a round
+  bool ok = true;
+  for (int i0 = threadIdx.x; i0 < items; i0 += kBatch * BS) {
+    unsigned todo = 0;
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k)
+      if (i0 + k * BS < items) todo |= 1u << k;
+    for (unsigned polls = 0; todo; ++polls) {
+      unsigned long long hi[kBatch], lo[kBatch];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k)
+        if ((todo >> k) & 1u)
+          asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                       : "=l"(hi[k]), "=l"(lo[k])
+                       : "l"((const char*)slot + 16 * (size_t)(i0 + k * BS))
+                       : "memory");
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k)
+        if (((todo >> k) & 1u) && (int)(hi[k] >> 32) == d && (int)(lo[k] >> 32) == d) {
+          to[i0 + k * BS] = DF{__uint_as_float((unsigned)hi[k]), __uint_as_float((unsigned)lo[k])};
+          todo &= ~(1u << k);
+        }
+      if (todo && (polls > limit || ((polls & 63u) == 63u && *((volatile int*)err) != 0))) {
+        atomicExch(err, 1);
+        ok = false;
+        break;
+      }
+    }
+  }
+  return ok;
+}
+
+// The block's total of sum q = lane & 7, in every lane of warp 0: lane groups
+// l>>3 = 0..3 each add four warps' sums, then two shuffle steps combine them.
+template <int NW>
+__device__ __forceinline__ DF block_total(const LsmShared<NW>& X) {
+  const int lane = threadIdx.x & 31, q = lane & 7;
   DF v = DF{X.wpart[lane >> 3][q], 0.f};
 #pragma unroll
   for (int w = (lane >> 3) + 4; w < NW; w += 4) v = df_add_f(v, X.wpart[w][q]);
   v = df_add(v, shfl_xor_df(v, 8));
-  v = df_add(v, shfl_xor_df(v, 16));
-  const int slot = d & 1;
-  const int G = P.nblocks;
-  DF g{0.f, 0.f};
-  if (MODE != kCoop) {
-    // Every CTA stores its eight totals into xin[slot][rank] of every CTA with
-    // st.async; each store counts its bytes against that CTA's xbar[slot],
-    // which the CTA's own lane 0 arms for G x 64 bytes (a store may land
-    // before the arming: the phase cannot complete before the arming's
-    // arrival). Slot reuse is safe: a CTA sends date d-2 only after its wait
-    // for date d-1, which needs every peer's date d-1 totals, which each peer
-    // sends after it has read its date d slot.
-    const int CL = MODE == kCluster ? G : P.cluster;
-    if (lane == 0) mbar_arrive_expect_tx(&X.xbar[slot], (uint32_t)(CL * kRegSums * sizeof(DF)));
-    if (lane < kRegSums) X.ctot[lane] = v;
-    __syncwarp();
-    if (lane < CL) {
-      const float4* src = reinterpret_cast<const float4*>(X.ctot);
-      const uint32_t dst = cluster_map(&X.xin[slot][rank][0], (uint32_t)lane);
-      const uint32_t bar = cluster_map(&X.xbar[slot], (uint32_t)lane);
+  return df_add(v, shfl_xor_df(v, 16));
+}
+
+// Sum over r = 0 .. n-1 of t[r][q], q = lane & 7, in every lane of a warp: lane
+// group l>>3 adds r = l>>3, l>>3 + 4, ... in that order. The next four are
+// loaded while four are added (the additions are one dependent chain); beyond
+// n a zero is added, which leaves a double-float as it is.
+__device__ __forceinline__ DF sum_totals(const DF* t, int n) {
+  const int lane = threadIdx.x & 31, q = lane & 7;
+  auto row = [&](int r) { return r < n ? t[r * kRegSums + q] : DF{0.f, 0.f}; };
+  DF g{0.f, 0.f}, x[4];
+  int r = lane >> 3;
 #pragma unroll
-      for (int j = 0; j < kRegSums * 2 / 4; ++j) st_async_v4(dst + 16u * j, src[j], bar);
-    }
-    if (!mbar_wait(&X.xbar[slot], (xph >> slot) & 1u, P.copy_wait_limit)) {
-      X.fail = 1;
-      atomicExch(P.err, 1);
-    }
-    xph ^= 1u << slot;
-    for (int r = lane >> 3; r < CL; r += 4) g = df_add(g, X.xin[slot][r][q]);
-    if (MODE == kCoopCluster) {
-      // Second level: every cluster now holds its total (the same bits in each
-      // of its CTAs); rank 0 publishes it, the clusters meet at a counter that
-      // grows by one arrival per cluster and date, and every CTA sums the
-      // cluster totals in cluster order.
-      g = df_add(g, shfl_xor_df(g, 8));
-      g = df_add(g, shfl_xor_df(g, 16));
-      const int ncl = G / CL, cid = b / CL;
-      float2* part = (float2*)P.partial + (size_t)slot * ncl * kRegSums;
-      if (rank == 0 && lane < kRegSums) {
-        part[(size_t)cid * kRegSums + lane] = make_float2(g.hi, g.lo);
-        __threadfence();
-      }
-      __syncwarp();
-      xcount += 1;
-      int ok = 1;
-      if (lane == 0) {
-        if (rank == 0) atomicAdd(P.barrier, 1u);
-        const unsigned target = xcount * (unsigned)ncl;
-        for (unsigned polls = 0;; ++polls) {
-          const unsigned cnt = *((volatile unsigned*)P.barrier);
-          if ((int)(cnt - target) >= 0) break;
-          if (*((volatile int*)P.err) != 0 || polls > P.wait_limit) {
-            atomicExch(P.err, 1);
-            ok = 0;
-            break;
-          }
-          __nanosleep(32);
-        }
-        __threadfence();
-      }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok && lane == 0) X.fail = 1;
-      g = DF{0.f, 0.f};
-#pragma unroll 4
-      for (int cc = lane >> 3; cc < ncl; cc += 4) {
-        const float2 p = __ldcg(part + (size_t)cc * kRegSums + q);
-        g = df_add(g, DF{p.x, p.y});
-      }
-    }
-  } else {
-    float2* part = (float2*)P.partial + (size_t)slot * G * kRegSums;
-    if (lane < kRegSums) {
-      part[(size_t)b * kRegSums + lane] = make_float2(v.hi, v.lo);
-      __threadfence();
-    }
-    __syncwarp();
-    int ok = 1;
-    if (lane == 0)
-      ok = group_arrive_wait(P.barrier, (unsigned)G + P.barrier_extra, P.err, P.wait_limit);
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    if (!ok && lane == 0) X.fail = 1;
-#pragma unroll 4
-    for (int bb = lane >> 3; bb < G; bb += 4) {
-      const float2 p = __ldcg(part + (size_t)bb * kRegSums + q);
-      g = df_add(g, DF{p.x, p.y});
+  for (int i = 0; i < 4; ++i) x[i] = row(r + 4 * i);
+#pragma unroll 1
+  for (int r0 = 0; r0 < n; r0 += 16) {
+    r += 16;
+    DF y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) y[i] = row(r + 4 * i);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      g = df_add(g, x[i]);
+      x[i] = y[i];
     }
   }
   g = df_add(g, shfl_xor_df(g, 8));
-  g = df_add(g, shfl_xor_df(g, 16));  // lanes 0..7: the contract's sum q = lane
+  return df_add(g, shfl_xor_df(g, 16));
+}
+
+// Exchange of the CTAs' totals within a cluster, by warp 0: every CTA stores
+// its eight totals into xin[slot][rank] of every CTA with st.async, lane (r, q)
+// the sum q to the CTAs r, r + 4, ...; each store counts its bytes against that
+// CTA's xbar[slot], which the CTA's own lane 0 arms for CL x 64 bytes (a store
+// may land before the arming: the phase cannot complete before the arming's
+// arrival). Slot reuse is safe: a CTA sends date d-2 only after its wait for
+// date d-1, which needs every peer's date d-1 totals, which each peer sends
+// after it has read its date d slot.
+template <int NW>
+__device__ __forceinline__ DF cluster_total(const LsmParams& P, LsmShared<NW>& X, DF v, int slot,
+                                            int rank, int CL, uint32_t& xph) {
+  const int lane = threadIdx.x & 31, q = lane & 7;
+  if (lane == 0) mbar_arrive_expect_tx(&X.xbar[slot], (uint32_t)(CL * kRegSums * sizeof(DF)));
+  for (int r = lane >> 3; r < CL; r += 4)
+    st_async_df(cluster_map(&X.xin[slot][rank][q], (uint32_t)r), v,
+                cluster_map(&X.xbar[slot], (uint32_t)r));
+  if (!mbar_wait(&X.xbar[slot], (xph >> slot) & 1u, P.copy_wait_limit)) {
+    X.fail = 1;
+    atomicExch(P.err, 1);
+  }
+  xph ^= 1u << slot;
+  DF g{0.f, 0.f};
+  for (int r = lane >> 3; r < CL; r += 4) g = df_add(g, X.xin[slot][r][q]);
+  g = df_add(g, shfl_xor_df(g, 8));
+  return df_add(g, shfl_xor_df(g, 16));
+}
+
+// Date d's normal equations from the contract's sums g (lane q's sum in every
+// lane q of each group of eight), by warp 0; leaves the mode and coefficients
+// in X.coef.
+template <int NW>
+__device__ __forceinline__ void solve_date(const LsmParams& P, LsmShared<NW>& X, DF g, int d, int b,
+                                           float growth) {
+  const int lane = threadIdx.x & 31;
+  const int q = lane & 7;
   if (q >= 5) g = df_mul(g, DF{growth, 0.f});  // y sums: cash flows grown to date d
   if (P.dbg_sums && b == 0 && lane < kRegSums) P.dbg_sums[(size_t)d * kRegSums + lane] = df_value(g);
   // include/common.h:98-141 solves the normal equations by the adjugate over
@@ -423,54 +436,75 @@ __device__ __forceinline__ void regress_date(const LsmParams& P, LsmShared<NW>& 
     const float s = __int_as_float((254 - e) << 23);  // 2^-(e - 127), exact
     g = DF{g.hi * s, g.lo * s};
   }
-  if (lane < kRegSums) X.tdf[lane] = g;
-  __syncwarp();
-  const DF* a = X.tdf;
-  DF cof{0.f, 0.f};
-  if (lane < 6) {
-    const int sh = 4 * lane;  // operand indices of cofactor `lane`, one nibble per lane
-    cof = df_add(df_mul(a[(0x010122 >> sh) & 15], a[(0x224334 >> sh) & 15]),
-                 df_neg(df_mul(a[(0x102213 >> sh) & 15], a[(0x132243 >> sh) & 15])));
-    X.cof[lane] = cof;
+  // Operand indices of cofactor `lane` (lanes 0..5; the other lanes' results
+  // are not used) and of row `lane` of the adjugate (row 0 again for lane 3),
+  // one nibble per lane; operands move between lanes by shuffles.
+  const int sh = 4 * q;
+  const DF o0 = shfl_df(g, (0x010122 >> sh) & 7), o1 = shfl_df(g, (0x224334 >> sh) & 7);
+  const DF o2 = shfl_df(g, (0x102213 >> sh) & 7), o3 = shfl_df(g, (0x132243 >> sh) & 7);
+  const int y0 = q < 3 ? 5 : 0;
+  const DF ya = shfl_df(g, y0), yb = shfl_df(g, y0 + 1), yc = shfl_df(g, y0 + 2);
+  const DF cof = df_add(df_mul(o0, o1), df_neg(df_mul(o2, o3)));
+  const DF k0 = shfl_df(cof, (0x0210 >> sh) & 7), k1 = shfl_df(cof, (0x1431 >> sh) & 7);
+  const DF k2 = shfl_df(cof, (0x2542 >> sh) & 7);
+  const DF dot = df_add(df_add(df_mul(k0, ya), df_mul(k1, yb)), df_mul(k2, yc));
+  const float det = __shfl_sync(0xffffffffu, dot.hi, 3);
+  int mode = 2;
+  if (n == 0.f) mode = 0;
+  else if (n <= 2.f) mode = 1;
+  else if (!(det > 0.f) || !(det < INFINITY)) mode = 3;  // include/common.h:115-117
+  float c = mode == 2 ? (dot.hi + dot.lo) * __frcp_rn(det) : 0.f;  // lanes 0..2
+  if (mode == 3) {
+    mode = 0;
+    if (b == 0 && lane == 0) atomicAdd(P.singular, 1);
   }
-  __syncwarp();
-  DF dot{0.f, 0.f};
-  if (lane < 4) {
-    const int sh = 4 * lane;  // adjugate row `lane` (row 0 again for lane 3)
-    const DF* y = lane < 3 ? a + 5 : a;
-    dot = df_add(df_add(df_mul(X.cof[(0x0210 >> sh) & 15], y[0]),
-                        df_mul(X.cof[(0x1431 >> sh) & 15], y[1])),
-                 df_mul(X.cof[(0x2542 >> sh) & 15], y[2]));
+  if (lane == 3) c = __int_as_float(mode);
+  if (lane < 4) X.coef[lane] = c;
+  if (P.dbg_coef && b == 0 && lane < 4)
+    P.dbg_coef[(size_t)d * 4 + (lane == 3 ? 0 : lane + 1)] = lane == 3 ? (float)mode : c;
+}
+
+// The totals that go through global memory: one per block, or one per cluster,
+// published by its rank 0 (the same bits in each of its CTAs).
+struct GlobalTotals {
+  DF* xs;     // shared memory they are gathered in
+  char* at;   // two slots by the date's parity
+  int n, me;  // how many, and the one this block publishes (-1: none)
+  __device__ GlobalTotals(const LsmParams& P, DF* to, int mode, int b, int rank)
+      : xs(to), at((char*)P.partial) {
+    n = mode == kCoopCluster ? P.nblocks / P.cluster : P.nblocks;
+    me = mode == kCoop ? b : mode == kCoopCluster && rank == 0 ? b / P.cluster : -1;
   }
-  const DF n1 = shfl_df(dot, 1), n2 = shfl_df(dot, 2), det = shfl_df(dot, 3);
-  if (lane == 0) {
-    int mode = 2;
-    float c0 = 0.f, c1 = 0.f, c2 = 0.f;
-    if (n == 0.f) {
-      mode = 0;
-    } else if (n <= 2.f) {
-      mode = 1;
-    } else if (!(det.hi > 0.f) || !(det.hi < INFINITY)) {  // include/common.h:115-117
-      mode = 0;
-      if (b == 0) atomicAdd(P.singular, 1);
-    } else {
-      const float r = 1.f / det.hi;
-      c0 = (dot.hi + dot.lo) * r;
-      c1 = (n1.hi + n1.lo) * r;
-      c2 = (n2.hi + n2.lo) * r;
-    }
-    X.mode = mode;
-    X.coef[0] = c0;
-    X.coef[1] = c1;
-    X.coef[2] = c2;
-    if (P.dbg_coef && b == 0) {
-      float* o = P.dbg_coef + (size_t)d * 4;
-      o[0] = (float)mode;
-      o[1] = c0;
-      o[2] = c1;
-      o[3] = c2;
-    }
+};
+
+// Date d's regression from the warps' sums in X.wpart, by the whole block
+// between two block barriers (the caller's): warp 0 forms the block's total,
+// the totals are exchanged, and warp 0 sums all of them in block order, so that
+// every block gets the same bits, and solves. `others` is what the warps that
+// do not sum have to do meanwhile.
+template <int MODE, int NW, typename Others>
+__device__ __forceinline__ void regress_date(const LsmParams& P, LsmShared<NW>& X,
+                                             const GlobalTotals& G, int d, int b, int rank,
+                                             uint32_t& xph, float growth, Others&& others) {
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, slot = d & 1;
+  DF g{0.f, 0.f};
+  if (wid == 0) {
+    g = block_total(X);
+    if (MODE == kCluster) g = cluster_total(P, X, g, slot, rank, P.nblocks, xph);
+    if (MODE == kCoopCluster) g = cluster_total(P, X, g, slot, rank, P.cluster, xph);
+  } else {
+    others();
   }
+  if (MODE != kCluster) {
+    char* part = G.at + (size_t)slot * (G.n + 1) * kRegSums * 16;
+    if (wid == 0 && lane < kRegSums && G.me >= 0) publish_total(part, G.me * kRegSums + lane, g, d);
+    // (test hook: one total more than there are, which nothing publishes)
+    const int items = G.n * kRegSums + (P.barrier_extra ? 1 : 0);
+    if (!gather_totals<NW * 32>(part, items, d, G.xs, P.err, P.wait_limit)) X.fail = 1;
+    __syncthreads();
+    if (wid == 0) g = sum_totals(G.xs, G.n);
+  }
+  if (wid == 0) solve_date(P, X, g, d, b, growth);
 }
 
 // Antithetic pairs p and p + 1 (p even; the second only if `two`) over the
@@ -589,6 +623,10 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
   const int M = P.M;
   const LsmSmem<TauT> S = carve<TauT>(smem_raw, PB, M);
   __shared__ LsmShared<BS / 32> X;
+  // Totals that come through global memory: in the cash flows' place, which is
+  // used only after the sweep, or behind everything (exchange_bytes).
+  const GlobalTotals G(P, exchange_fits(PB, P.nblocks) ? (DF*)S.cf : (DF*)(S.buf + (size_t)4 * PB),
+                       MODE, b, rank);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 
   const long long p0 = (long long)b * PB;
@@ -647,10 +685,11 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
   }
 
   // Buffer schedule: date d's slice sits in buf[(M - 1 - d) & 1]. Thread 32
-  // issues every copy; every thread waits on the copy it is about to read.
-  // `pend` (copies issued, not yet waited) and `ph` (mbarrier parities) evolve
-  // the same way in every thread.
-  uint32_t ph = 0, pend = 0, xph = 0, xcount = 0;
+  // issues every copy. All warps but the first wait for the slice they read
+  // next while the first one exchanges and solves; the block barrier after that
+  // covers warp 0. `pend` (copies issued, not yet waited) and `ph` (mbarrier
+  // parities) evolve the same way in every thread.
+  uint32_t ph = 0, pend = 0, xph = 0;
   if (nbr > 0) {
     if (threadIdx.x == 32) {
       issue_row(P, M - 2, p0, nbr, PB, S.slice(0), &S.bar[0]);                 // date M-1
@@ -659,26 +698,33 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
     pend = M >= 3 ? 3u : 1u;
   }
   auto wait_copy = [&](int k) {
-    if (!((pend >> k) & 1u)) return;
     if (!mbar_wait(&S.bar[k], (ph >> k) & 1u, P.copy_wait_limit)) {
       X.fail = 1;
       atomicExch(P.err, 2);
     }
+  };
+  auto waited = [&](int k) {
     ph ^= 1u << k;
     pend &= ~(1u << k);
   };
-  // Regression for date d from each thread's sums; then thread 32 issues the
-  // copy of `next_row` into buf[next_k] (free: every thread has passed the
-  // first barrier, so it is done reading that buffer).
-  auto regress = [&](const float (&acc)[kRegSums], int d, int next_row, int next_k) {
+  // Regression for date d from each thread's sums. Date d's slice has been read
+  // (its values are in registers), so thread 32 issues the copy of date d - 2
+  // into its buffer, a whole date before it is read; the slice of date d - 1 is
+  // waited for.
+  auto regress = [&](const float (&acc)[kRegSums], int d) {
     const float v = warp_scatter8(acc);
     if ((lane & 3) == 0) X.wpart[wid][lane >> 2] = v;
     __syncthreads();
-    if (next_row >= 0 && nbr > 0) {
-      if (threadIdx.x == 32) issue_row(P, next_row, p0, nbr, PB, S.slice(next_k), &S.bar[next_k]);
-      pend |= 1u << next_k;
+    const int kd = (M - 1 - d) & 1, kn = kd ^ 1;
+    if (d >= 3 && nbr > 0) {
+      if (threadIdx.x == 32) issue_row(P, d - 3, p0, nbr, PB, S.slice(kd), &S.bar[kd]);
+      pend |= 1u << kd;
     }
-    if (wid == 0) regress_date<MODE, BS / 32>(P, X, d, b, rank, xph, xcount, S.edt[d]);
+    const bool wait = d > 1 && ((pend >> kn) & 1u);
+    regress_date<MODE, BS / 32>(P, X, G, d, b, rank, xph, S.edt[d], [&]() {
+      if (wait) wait_copy(kn);
+    });
+    if (wait) waited(kn);
     __syncthreads();
   };
 
@@ -702,13 +748,16 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
 
   // Sums for date M-1 (the only date without a preceding update pass).
   {
-    wait_copy(0);
+    if (pend & 1u) {
+      wait_copy(0);
+      waited(0);
+    }
     float acc[kRegSums];
 #pragma unroll
     for (int q = 0; q < kRegSums; ++q) acc[q] = 0.f;
 #pragma unroll
     for (int k = 0; k < J; ++k) gather(S.slice(0), k, acc);
-    regress(acc, M - 1, -1, 0);
+    regress(acc, M - 1);
   }
 
   // Date m: update with date m's coefficients, fused with the sums of date m-1.
@@ -716,9 +765,9 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
   for (int m = M - 1; m >= 1 && !failed; --m) {
     const int kb = (M - 1 - m) & 1;
     const bool has_next = m > 1;
-    if (has_next) wait_copy(kb ^ 1);
-    const int mode = X.mode;
-    const float c0 = X.coef[0], c1 = X.coef[1], c2 = X.coef[2];
+    const float4 fit = ld4(X.coef);
+    const int mode = __float_as_int(fit.w);
+    const float c0 = fit.x, c1 = fit.y, c2 = fit.z;
     const float dm = S.dt[m], em = S.edt[m];
     const float* nxt = S.slice(kb ^ 1);
     float acc[kRegSums];
@@ -780,7 +829,7 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
       else if (mode == 2) sweep(Md2{}, No{}, No{});
     }
     if (!has_next) break;
-    regress(acc, m - 1, m - 2 >= 1 ? m - 3 : -1, kb);
+    regress(acc, m - 1);
     failed = !DSMEM && X.fail;
   }
   if (!failed)  // the final sums go over the pairs in another order
@@ -889,6 +938,7 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_stream_kernel(LsmParams P) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   float* dt = stab;
   float* edt = stab + (M + 1);
+  const GlobalTotals G(P, (DF*)(stab + ((2 * (M + 1) + 3) & ~3)), kCoop, b, 0);
   const long long PB = P.pairs_per_block, Hp = P.Hp;
   const long long p0 = (long long)b * PB;
   const long long nb = max(0LL, min(PB, P.H - p0));
@@ -917,12 +967,12 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_stream_kernel(LsmParams P) {
   }
   __syncthreads();  // every path of the block is read below by another thread
 
-  uint32_t xph = 0, xcount = 0;
+  uint32_t xph = 0;
   auto regress = [&](const float (&acc)[kRegSums], int d) {
     const float v = warp_scatter8(acc);
     if ((lane & 3) == 0) X.wpart[wid][lane >> 2] = v;
     __syncthreads();
-    if (wid == 0) regress_date<kCoop, NW>(P, X, d, b, 0, xph, xcount, edt[d]);
+    regress_date<kCoop, NW>(P, X, G, d, b, 0, xph, edt[d], []() {});
     __syncthreads();
   };
   {
@@ -947,8 +997,9 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_stream_kernel(LsmParams P) {
   bool failed = X.fail;
   for (int m = M - 1; m >= 1 && !failed; --m) {
     const bool has_next = m > 1;
-    const int mode = X.mode;
-    const float c0 = X.coef[0], c1 = X.coef[1], c2 = X.coef[2];
+    const float4 fit = ld4(X.coef);
+    const int mode = __float_as_int(fit.w);
+    const float c0 = fit.x, c1 = fit.y, c2 = fit.z;
     const float dm = dt[m], em = edt[m];
     const float* cur = P.paths + (size_t)(m - 1) * stride + p0;  // date m is row m-1
     const float* nxt = has_next ? cur - stride : cur;
@@ -1087,6 +1138,9 @@ size_t lsm_smem(int PB, int M, size_t tau_bytes) {
 }
 
 size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// The exchange buffer of a cooperative contract of at most G blocks.
+size_t totals_bytes(int G) { return 2 * ((size_t)G + 1) * kRegSums * 16; }
 
 // Parameters of one contract that do not depend on where its buffers live.
 void lsm_fill(LsmParams& P, double S0, double E, double r, double sigma, double T, long long N,
@@ -1228,14 +1282,15 @@ bool coop_shape(const pcf_ctx* c, const LsmLimits& Lm, long long H, int M, int& 
                                               (long long)c->sm_count));
   PB = (int)((((H + G0 - 1) / G0) + 3) & ~3LL);
   G = (int)((H + PB - 1) / PB);
-  smem = lsm_smem(PB, M, 2);
+  smem = lsm_smem(PB, M, 2) + exchange_bytes(PB, G);
   return lsm_fits(Lm, PB, M, 2, Lm.stat_coop, 1);
 }
 
 // Grid of the streaming sweep (lsm_stream_kernel) for a contract of H pairs:
 // one block per SM (cooperative), the pairs split evenly in multiples of 4.
 int stream_shape(const pcf_ctx* c, long long H, int M, int& G, int& PB, size_t& smem) {
-  smem = sizeof(float) * 2 * (size_t)(M + 1);
+  smem = r16(sizeof(float) * 2 * (size_t)(M + 1)) +
+         ((size_t)c->sm_count + 1) * kRegSums * sizeof(DF);
   int occ = 0;
   const int st = cuda_status(
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, lsm_stream_kernel, kLsmBlock, smem),
@@ -1314,7 +1369,7 @@ int launch_coop(const LsmParams& P0, int G, int PB, size_t smem, int hcl, int Gh
     at[1].val.cooperative = 1;
     cfg.gridDim = dim3(Gh);
     cfg.blockDim = dim3(kLsmBlock);
-    cfg.dynamicSmemBytes = lsm_smem(PBh, P.M, 2);
+    cfg.dynamicSmemBytes = lsm_smem(PBh, P.M, 2) + exchange_bytes(PBh, Gh);
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 2;
@@ -1442,6 +1497,8 @@ int group_of(int cl, int k, bool t8) {
   return (lg * kNumPB + k) * 2 + (t8 ? 1 : 0);
 }
 
+constexpr size_t kCoopZero = 256;  // the final reduction's ticket, ahead of the totals
+
 int lsm_layout(pcf_ctx* c, const std::vector<LsmRequest>& reqs, LsmLayout& L) {
   const LsmLimits& Lm = lsm_limits(c);
   if (Lm.status) return Lm.status;
@@ -1490,8 +1547,8 @@ int lsm_layout(pcf_ctx* c, const std::vector<LsmRequest>& reqs, LsmLayout& L) {
       L.stream[i] = 1;
     }
     const size_t gm = (size_t)std::max(L.coop_G[i], L.coop_Gh[i]);
-    L.o_coop[i] = off;  // partial (2 G 8 float2) | fpartial (G 5 float2) | 2 counters
-    off = a256(off + 8 * (2 * gm * kRegSums + gm * kMoments) + 16);
+    L.o_coop[i] = off;  // ticket | exchanged totals (both 0 at launch) | fpartial (G 5 float2)
+    off = a256(off + kCoopZero + totals_bytes((int)gm) + 8 * gm * kMoments);
   }
   L.o_paths.assign(n, 0);
   for (size_t i = 0; i < n; ++i) {
@@ -1586,11 +1643,9 @@ int lsm_batch_create(pcf_ctx* c, const std::vector<LsmRequest>& reqs, cudaStream
     P.nblocks = Lo.coop_G[i];
     const size_t gm = (size_t)std::max(Lo.coop_G[i], Lo.coop_Gh[i]);
     char* base = d + Lo.o_coop[i];
-    P.partial = (double*)base;
-    P.fpartial = (double*)(base + 8 * 2 * gm * kRegSums);
-    unsigned* cnt = (unsigned*)(base + 8 * (2 * gm * kRegSums + gm * kMoments));
-    P.barrier = cnt;
-    P.ticket = cnt + 1;
+    P.ticket = (unsigned*)base;
+    P.partial = (double*)(base + kCoopZero);
+    P.fpartial = (double*)(base + kCoopZero + totals_bytes((int)gm));
     if (Lo.stream[i]) {
       const size_t mb = a256(sizeof(float) * (size_t)P.M * 2 * (size_t)P.Hp);
       P.gcf = (float*)(d + Lo.o_paths[i] + mb);
@@ -1649,7 +1704,8 @@ int lsm_batch_launch_coop(pcf_ctx* c, LsmBatch* B, cudaStream_t s) {
   int st;
   for (size_t i = 0; i < B->coop.size(); ++i) {
     LsmParams& P = B->coop[i];
-    st = cuda_status(cudaMemsetAsync(P.barrier, 0, 2 * sizeof(unsigned), s), "memset LSM counters");
+    const size_t zero = (size_t)((char*)P.fpartial - (char*)P.ticket);
+    st = cuda_status(cudaMemsetAsync(P.ticket, 0, zero, s), "memset LSM exchange");
     if (st) return st;
     if (B->coop_stream[i]) {
       P.pairs_per_block = B->coop_pb[i];
@@ -1748,11 +1804,12 @@ int amer_run(pcf_ctx* ctx, double S0, double E, double r, double sigma, double T
     if (st) return st;
     c->paths_cap = paths_bytes;
   }
-  // Scratch: dtab | partial | fpartial | counters | out [| audit coef | sums | tau].
+  // Scratch: dtab | fpartial | exchanged totals | counters | out
+  // [| audit coef | sums | tau]. The totals and the counters are 0 at launch.
   const size_t o_dt = 0;
-  const size_t o_part = a256(o_dt + dtab_bytes(M));
-  const size_t o_fpart = a256(o_part + sizeof(double) * 2 * Gmax * kRegSums);
-  const size_t o_cnt = a256(o_fpart + sizeof(double) * Gmax * kMoments);
+  const size_t o_fpart = a256(o_dt + dtab_bytes(M));
+  const size_t o_part = a256(o_fpart + sizeof(double) * Gmax * kMoments);
+  const size_t o_cnt = a256(o_part + totals_bytes(Gmax));
   const size_t o_out = a256(o_cnt + sizeof(unsigned) * 4);
   const size_t o_acoef = a256(o_out + sizeof(double) * kMoments);
   const size_t o_asums = a256(o_acoef + (au ? sizeof(float) * 4 * (size_t)M : 0));
@@ -1765,7 +1822,7 @@ int amer_run(pcf_ctx* ctx, double S0, double E, double r, double sigma, double T
   dtab_fill((float*)(h + o_dt), r, T, M);
   st = cuda_status(cudaMemcpyAsync(d + o_dt, h + o_dt, dtab_bytes(M), cudaMemcpyHostToDevice,
                                    c->stream), "H2D dtab");
-  if (!st) st = cuda_status(cudaMemsetAsync(d + o_cnt, 0, sizeof(unsigned) * 4, c->stream),
+  if (!st) st = cuda_status(cudaMemsetAsync(d + o_part, 0, o_out - o_part, c->stream),
                             "memset counters");
   if (!st && au)  // dates without a regression (date 0, skipped dates) read as mode 0
     st = cuda_status(cudaMemsetAsync(d + o_acoef, 0, total - o_acoef, c->stream), "memset audit");
@@ -1775,7 +1832,6 @@ int amer_run(pcf_ctx* ctx, double S0, double E, double r, double sigma, double T
   P.partial = (double*)(d + o_part);
   P.fpartial = (double*)(d + o_fpart);
   unsigned* cnt = (unsigned*)(d + o_cnt);
-  P.barrier = cnt;
   P.ticket = cnt + 1;
   P.err = (int*)(cnt + 2);
   P.singular = (int*)(cnt + 3);

@@ -423,16 +423,15 @@ __device__ __forceinline__ uint32_t cluster_map(const void* p, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
   return r;
 }
-// Asynchronous store of 16 bytes into another CTA's shared memory; its
-// completion counts 16 bytes against that CTA's mbarrier (complete_tx), so
-// the sender needs no fence and the receiver sees the data once the phase
-// completes.
-__device__ __forceinline__ void st_async_v4(uint32_t addr, float4 v, uint32_t bar) {
-  asm volatile(
-      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, "
-      "[%5];" ::"r"(addr),
-      "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
-      : "memory");
+// Asynchronous store of a double-float into another CTA's shared memory; its
+// completion counts 8 bytes against that CTA's mbarrier (complete_tx), so the
+// sender needs no fence and the receiver sees the data once the phase completes.
+__device__ __forceinline__ void st_async_df(uint32_t addr, DF v, uint32_t bar) {
+  const unsigned long long x =
+      (unsigned long long)__float_as_uint(v.hi) | ((unsigned long long)__float_as_uint(v.lo) << 32);
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+               "l"(x), "r"(bar)
+               : "memory");
 }
 
 // Group barrier for a persistent kernel whose blocks are co-resident (the

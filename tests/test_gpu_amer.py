@@ -325,3 +325,38 @@ def test_context_release_and_memory_limit(ctx):
     ctx.set_memory_limit(0)
     again = mc_amer_result(*args, seed=8, ctx=ctx)
     assert list(again.sums) == list(first.sums)
+
+
+@pytest.mark.parametrize("N,M", [(2, 3), (10, 2), (1026, 3), (1030, 12), (64514, 7), (100_002, 10),
+                                 (310_000, 5), (700_002, 5), (1_400_002, 4)])
+def test_amer_slices_and_exchange_match_fp64_twin(orc, ctx, N, M):
+    """Cooperative launches whose slices and exchanges differ: one block, two
+    blocks with a ragged last group, 64 blocks of 508 pairs (the totals do not
+    fit in the cash flows' place), one, two and four groups of pairs a thread,
+    with and without clusters; 2 to 12 dates, so that the copies a date ahead
+    start and end early. The module's bar for puts; a handful of paths decides
+    on exact ties only, so its sums agree to FP32."""
+    from parcompfin_gb300 import mc_amer_result
+    res = mc_amer_result(100, 104, .05, .3, 1.0, N, M, -1, seed=5, ctx=ctx)
+    s = twin(orc, 100, 104, .05, .3, 1.0, N, M, -1, 0, 5)
+    assert s[5] == 0
+    for k in (0, 2):
+        assert abs(res.sums[k] - s[k]) <= 3e-4 * abs(s[k]), (k, res.sums[k], s[k])
+
+
+@pytest.mark.parametrize("N,M", [(1024, 5), (4100, 7), (16_386, 6), (65_536, 9), (131_074, 300),
+                                 (262_144, 6)])
+def test_amer_batch_slices_match_fp64_twin(orc, ctx, N, M):
+    """Cluster launches over slices of 512 to 8192 pairs (one, two and four
+    groups of pairs a thread), 8- and 16-bit exercise dates, a ragged last CTA;
+    the same contract alone and among others gives the same bits."""
+    import parcompfin_gb300 as pcf
+    q = pcf.request("amer", 100, 104, .05, .3, 1.0, N, "put", M=M, seed=5, use_cv=True, stream=0)
+    others = [pcf.request("amer", 100, 95 + k, .05, .3, 1.0, 2048, "put", M=10, seed=6, stream=k)
+              for k in range(3)]
+    res = pcf.price_batch([q], ctx=ctx)[0]
+    assert list(res.sums) == list(pcf.price_batch(others + [q], ctx=ctx)[3].sums)
+    s = twin(orc, 100, 104, .05, .3, 1.0, N, M, -1, 0, 5)
+    assert s[5] == 0
+    for k in (0, 2):
+        assert abs(res.sums[k] - s[k]) <= 3e-4 * abs(s[k]), (k, res.sums[k], s[k])
