@@ -60,50 +60,91 @@ __device__ __forceinline__ float payoff(const McContract& C, float S) {
 
 // European: item j covers path quads [j*U, (j+1)*U), U = units_per_item.
 // Quad q's four paths take the four normals of Philox block (x=q, y=0).
-// S_T = 2^(log2 S0 + a2 + b2 z); y = payoff(S_T), g = S_T.
+// S_T = 2^(log2 S0 + a2 + b2 z); y = payoff(S_T), g = S_T. Sums of four quads
+// are added in FP32, then with compensation.
+struct EurSums {
+  float cy = 0.f, cyy = 0.f, cg = 0.f, cgg = 0.f, cyg = 0.f;
+};
+
+// One quad's paths from its words; the first `left` of them count.
+template <bool CV, bool PART>
+__device__ __forceinline__ void eur_quad(const McContract& C, float a2, uint4 w, int left,
+                                         EurSums& c) {
+  const float4 z = normals4_x2(w);
+  // Paths (0, 2) and (1, 3) side by side in packed FP32x2 arithmetic
+  // (each lane rounds exactly as the scalar operation).
+  const float2 b2 = make_float2(C.b2, C.b2), a22 = make_float2(a2, a2);
+  const float2 e02 = __ffma2_rn(b2, make_float2(z.x, z.z), a22);
+  const float2 e13 = __ffma2_rn(b2, make_float2(z.y, z.w), a22);
+  const float2 s02 = make_float2(ex2_approx(e02.x), ex2_approx(e02.y));
+  const float2 s13 = make_float2(ex2_approx(e13.x), ex2_approx(e13.y));
+  const float2 pf = make_float2(C.pf, C.pf), nK = make_float2(C.nK, C.nK);
+  const float2 v02 = __ffma2_rn(pf, s02, nK), v13 = __ffma2_rn(pf, s13, nK);
+  float s[4] = {s02.x, s13.x, s02.y, s13.y};
+  float y[4] = {fmaxf(v02.x, 0.f), fmaxf(v13.x, 0.f), fmaxf(v02.y, 0.f),
+                fmaxf(v13.y, 0.f)};  // payoff
+  if (PART) {
+#pragma unroll
+    for (int l = 0; l < 4; ++l)
+      if (l >= left) y[l] = s[l] = 0.f;
+  }
+  c.cy += (y[0] + y[1]) + (y[2] + y[3]);
+  c.cyy = fmaf(y[0], y[0], fmaf(y[1], y[1], fmaf(y[2], y[2], fmaf(y[3], y[3], c.cyy))));
+  if (CV) {
+    c.cg += (s[0] + s[1]) + (s[2] + s[3]);
+    c.cgg = fmaf(s[0], s[0], fmaf(s[1], s[1], fmaf(s[2], s[2], fmaf(s[3], s[3], c.cgg))));
+    c.cyg = fmaf(y[0], s[0], fmaf(y[1], s[1], fmaf(y[2], s[2], fmaf(y[3], s[3], c.cyg))));
+  }
+}
+
 template <bool CV, int BS>
 __device__ __forceinline__ void eur_item(const McContract& C, int j, Moments<CV>& mo) {
-  const long long nq = (C.N + 3) >> 2;
-  const long long nfull = C.N >> 2;  // quads whose four paths are all < N
-  const long long q0 = (long long)j * C.units_per_item + threadIdx.x;
+  const long long first = (long long)j * C.units_per_item;
   const int qpt = C.units_per_item / BS;
   const RngKey key{C.seed_lo, C.seed_hi, C.stream, TAG_EUR};
   const float a2 = C.a2 + C.l2S0;
-  for (int k0 = 0; k0 < qpt; k0 += 4) {
-    float cy = 0.f, cyy = 0.f, cg = 0.f, cgg = 0.f, cyg = 0.f;
+  const uint64_t x0 = (uint64_t)(C.x0 + first);
+  const bool one_word = (uint32_t)x0 <= 0xffffffffu - (uint32_t)C.units_per_item;
+  if (first + C.units_per_item <= (C.N >> 2) && one_word && (qpt & 3) == 0) {
+    // Every quad is whole and their numbers differ in the low word only: no
+    // test and no 64-bit arithmetic a quad.
+    const uint32_t hi = (key.tag << 16) | ((uint32_t)(x0 >> 32) & 0xffffu);
+    // Consecutive quads of a thread differ by BS, so the first round's product
+    // M0 x grows by a constant, and round 2's product of word x is the
+    // contract's: 17.5 of the 20 products are left.
+    uint64_t p = (uint64_t)((uint32_t)x0 + threadIdx.x) * kPhiloxM0;
+    uint32_t hs, ls, h0, l0;
+    mul_wide(key.stream, kPhiloxM1, hs, ls);
+    mul_wide(hs ^ key.k0, kPhiloxM0, h0, l0);
+    const uint32_t k0b = key.k0 + kPhiloxW0, k1b = key.k1 + kPhiloxW1;
+    const uint32_t hk = hi ^ key.k1, lk = ls ^ k0b, hk2 = h0 ^ k1b;
+#pragma unroll 1
+    for (int k0 = 0; k0 < qpt; k0 += 4) {
+      EurSums c;
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      const long long q = q0 + (long long)(k0 + kk) * BS;
-      if (k0 + kk < qpt && q < nq) {
-        const float4 z = normals4_x2(draw_words(key, (uint64_t)(C.x0 + q), 0u));
-        // Paths (0, 2) and (1, 3) side by side in packed FP32x2 arithmetic
-        // (each lane rounds exactly as the scalar operation).
-        const float2 b2 = make_float2(C.b2, C.b2), a22 = make_float2(a2, a2);
-        const float2 e02 = __ffma2_rn(b2, make_float2(z.x, z.z), a22);
-        const float2 e13 = __ffma2_rn(b2, make_float2(z.y, z.w), a22);
-        const float2 s02 = make_float2(ex2_approx(e02.x), ex2_approx(e02.y));
-        const float2 s13 = make_float2(ex2_approx(e13.x), ex2_approx(e13.y));
-        const float2 pf = make_float2(C.pf, C.pf), nK = make_float2(C.nK, C.nK);
-        const float2 v02 = __ffma2_rn(pf, s02, nK), v13 = __ffma2_rn(pf, s13, nK);
-        float s[4] = {s02.x, s13.x, s02.y, s13.y};
-        float y[4] = {fmaxf(v02.x, 0.f), fmaxf(v13.x, 0.f), fmaxf(v02.y, 0.f),
-                      fmaxf(v13.y, 0.f)};  // payoff
-        if (q >= nfull) {  // the one partial quad at the end of the contract
-          const long long left = C.N - 4 * q;
-#pragma unroll
-          for (int l = 0; l < 4; ++l)
-            if (l >= left) y[l] = s[l] = 0.f;
-        }
-        cy += (y[0] + y[1]) + (y[2] + y[3]);
-        cyy = fmaf(y[0], y[0], fmaf(y[1], y[1], fmaf(y[2], y[2], fmaf(y[3], y[3], cyy))));
-        if (CV) {
-          cg += (s[0] + s[1]) + (s[2] + s[3]);
-          cgg = fmaf(s[0], s[0], fmaf(s[1], s[1], fmaf(s[2], s[2], fmaf(s[3], s[3], cgg))));
-          cyg = fmaf(y[0], s[0], fmaf(y[1], s[1], fmaf(y[2], s[2], fmaf(y[3], s[3], cyg))));
-        }
+      for (int k = 0; k < 4; ++k, p += (uint64_t)BS * kPhiloxM0) {
+        uint32_t h, l;
+        mul_wide((uint32_t)(p >> 32) ^ hk, kPhiloxM1, h, l);
+        const uint4 w = philox_rounds<8>(make_uint4(h ^ lk, l, hk2 ^ (uint32_t)p, l0),
+                                         k0b + kPhiloxW0, k1b + kPhiloxW1);
+        eur_quad<CV, false>(C, a2, w, 4, c);
       }
+      mo.flush(c.cy, c.cyy, c.cg, c.cgg, c.cyg);
     }
-    mo.flush(cy, cyy, cg, cgg, cyg);
+    return;
+  }
+  const long long nq = (C.N + 3) >> 2;
+#pragma unroll 1
+  for (int k0 = 0; k0 < qpt; k0 += 4) {
+    EurSums c;
+#pragma unroll 1
+    for (int k = k0; k < min(k0 + 4, qpt); ++k) {
+      const long long q = first + threadIdx.x + (long long)k * BS;
+      if (q < nq)
+        eur_quad<CV, true>(C, a2, draw_words(key, (uint64_t)(C.x0 + q), 0u),
+                           (int)min(4LL, C.N - 4 * q), c);
+    }
+    mo.flush(c.cy, c.cyy, c.cg, c.cgg, c.cyg);
   }
 }
 
@@ -176,27 +217,31 @@ __device__ __forceinline__ void asia_step2(const McContract& C, float2 w2, float
 }
 
 // Two Asian paths at once (asia_path for paths n0 and n1, the same bits),
-// their moments added in path order.
+// their moments added in path order. The steps are bound by the FMA pipe (the
+// Philox products, 149 of its 210 busy cycles per two paths and four steps of
+// 268) and by MUFU (162).
 template <int MODE, bool CV>
 __device__ __forceinline__ void asia_path2(const McContract& C, const RngKey& key, long long n0,
                                            long long n1, float w, Moments<CV>& mo) {
   const int M = C.M, Mfull = M & ~3;
   const float2 w2 = make_float2(w, w);
-  float2 L = make_float2(0.f, 0.f), I = L, lg = L;
+  float2 L = make_float2(0.f, 0.f), I = L, lg = L, z[4];
+  const PhiloxX x0 = philox_x(key, (uint64_t)(C.x0 + n0)), x1 = philox_x(key, (uint64_t)(C.x0 + n1));
+  auto draw = [&](int m0) {
+    const PhiloxY y = philox_y(key, (uint32_t)(m0 >> 2));
+    normals4_pair(draw_words(key, x0, y), draw_words(key, x1, y), z);
+  };
+#pragma unroll 1
   for (int m0 = 0; m0 < Mfull; m0 += 4) {
-    const float4 z0 = normals4_x2(draw_words(key, (uint64_t)(C.x0 + n0), (uint32_t)(m0 >> 2)));
-    const float4 z1 = normals4_x2(draw_words(key, (uint64_t)(C.x0 + n1), (uint32_t)(m0 >> 2)));
-    asia_step2<MODE, CV>(C, w2, make_float2(z0.x, z1.x), L, I, lg);
-    asia_step2<MODE, CV>(C, w2, make_float2(z0.y, z1.y), L, I, lg);
-    asia_step2<MODE, CV>(C, w2, make_float2(z0.z, z1.z), L, I, lg);
-    asia_step2<MODE, CV>(C, w2, make_float2(z0.w, z1.w), L, I, lg);
+    draw(m0);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) asia_step2<MODE, CV>(C, w2, z[l], L, I, lg);
   }
   if (Mfull < M) {
-    const float4 z0 = normals4_x2(draw_words(key, (uint64_t)(C.x0 + n0), (uint32_t)(Mfull >> 2)));
-    const float4 z1 = normals4_x2(draw_words(key, (uint64_t)(C.x0 + n1), (uint32_t)(Mfull >> 2)));
-    asia_step2<MODE, CV>(C, w2, make_float2(z0.x, z1.x), L, I, lg);
-    if (Mfull + 1 < M) asia_step2<MODE, CV>(C, w2, make_float2(z0.y, z1.y), L, I, lg);
-    if (Mfull + 2 < M) asia_step2<MODE, CV>(C, w2, make_float2(z0.z, z1.z), L, I, lg);
+    draw(Mfull);
+    asia_step2<MODE, CV>(C, w2, z[0], L, I, lg);
+    if (Mfull + 1 < M) asia_step2<MODE, CV>(C, w2, z[1], L, I, lg);
+    if (Mfull + 2 < M) asia_step2<MODE, CV>(C, w2, z[2], L, I, lg);
   }
   if (CV && MODE == 0) lg = __ffma2_rn(make_float2(C.w_last - w, C.w_last - w), L, lg);
   const float sw = C.S0 * w;

@@ -24,30 +24,82 @@ struct RngKey {
   uint32_t k0, k1, stream, tag;
 };
 
-__device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint32_t k0, uint32_t k1) {
+// The high and low words of a 32 x 32-bit product by one widening multiply, 4.8
+// cycles of an SM quarter's FMA pipe. These products are the largest part of the
+// Monte Carlo kernels' work on that pipe, which the FP32 arithmetic shares.
+__device__ __forceinline__ void mul_wide(uint32_t a, uint32_t b, uint32_t& hi, uint32_t& lo) {
+  asm("{\n\t.reg .u64 t;\n\tmul.wide.u32 t, %2, %3;\n\tmov.b64 {%1, %0}, t;\n\t}"
+      : "=r"(hi), "=r"(lo)
+      : "r"(a), "r"(b));
+}
+
+constexpr uint32_t kPhiloxM0 = 0xD2511F53u, kPhiloxM1 = 0xCD9E8D57u;
+constexpr uint32_t kPhiloxW0 = 0x9E3779B9u, kPhiloxW1 = 0xBB67AE85u;
+
+// R Philox rounds whose first uses the key (k0, k1).
+template <int R>
+__device__ __forceinline__ uint4 philox_rounds(uint4 c, uint32_t k0, uint32_t k1) {
 #pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    // The high and low words as two 32-bit multiplies (the same values as
-    // one 64-bit product; measured 1 % faster on the Asian book).
-    const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
-    const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
+  for (int r = 0; r < R; ++r) {
+    uint32_t hi0, lo0, hi1, lo1;
+    mul_wide(c.x, kPhiloxM0, hi0, lo0);
+    mul_wide(c.z, kPhiloxM1, hi1, lo1);
     c = make_uint4(hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0);
-    k0 += 0x9E3779B9u;
-    k1 += 0xBB67AE85u;
+    k0 += kPhiloxW0;
+    k1 += kPhiloxW1;
   }
   return c;
 }
 
+// One block. The basket kernels and the Longstaff-Schwartz forward pass, whose
+// registers are full, measured 1 to 5 % slower with mul_wide's register pairs
+// (basket book 720 -> 758 us), so the compiler chooses here.
 __device__ __forceinline__ uint4 draw_words(const RngKey& k, uint64_t x, uint32_t y) {
-  return philox4x32_10(
-      make_uint4((uint32_t)x, y, k.stream, (k.tag << 16) | ((uint32_t)(x >> 32) & 0xffffu)),
-      k.k0, k.k1);
+  uint4 c = make_uint4((uint32_t)x, y, k.stream, (k.tag << 16) | ((uint32_t)(x >> 32) & 0xffffu));
+  uint32_t k0 = k.k0, k1 = k.k1;
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    const uint32_t hi0 = __umulhi(kPhiloxM0, c.x), lo0 = kPhiloxM0 * c.x;
+    const uint32_t hi1 = __umulhi(kPhiloxM1, c.z), lo1 = kPhiloxM1 * c.z;
+    c = make_uint4(hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0);
+    k0 += kPhiloxW0;
+    k1 += kPhiloxW1;
+  }
+  return c;
 }
 
-// u = (2*(w >> 9) + 1) * 2^-24, exactly: 1.m - (1 - 2^-24) is an exact
-// subtraction (Sterbenz), so no integer-to-float conversion is needed.
-__device__ __forceinline__ float uniform_open(uint32_t w) {
-  return __uint_as_float(0x3f800000u | (w >> 9)) - 0.99999994f;
+// draw_words for many y at a fixed x: what the first three rounds make of x
+// alone (PhiloxX, once a path) and of y alone (PhiloxY, shared by the paths of
+// a thread), so that a block costs 7.5 of its 10 rounds.
+struct PhiloxX {
+  uint32_t a, b, h, l;
+};
+struct PhiloxY {
+  uint32_t h, l;
+};
+__device__ __forceinline__ PhiloxX philox_x(const RngKey& k, uint64_t x) {
+  uint32_t hs, ls, h0, l0, h, l;
+  PhiloxX r;
+  mul_wide(k.stream, kPhiloxM1, hs, ls);
+  mul_wide((uint32_t)x, kPhiloxM0, h0, l0);
+  mul_wide(h0 ^ ((k.tag << 16) | ((uint32_t)(x >> 32) & 0xffffu)) ^ k.k1, kPhiloxM1, h, l);
+  r.a = l0 ^ (k.k1 + kPhiloxW1);
+  r.b = l ^ (k.k0 + 2 * kPhiloxW0);
+  mul_wide(h ^ ls ^ (k.k0 + kPhiloxW0), kPhiloxM0, h, l);
+  r.h = h ^ (k.k1 + 2 * kPhiloxW1);
+  r.l = l;
+  return r;
+}
+__device__ __forceinline__ PhiloxY philox_y(const RngKey& k, uint32_t y) {
+  PhiloxY r;
+  mul_wide(__umulhi(k.stream, kPhiloxM1) ^ y ^ k.k0, kPhiloxM0, r.h, r.l);
+  return r;
+}
+__device__ __forceinline__ uint4 draw_words(const RngKey& k, const PhiloxX& x, const PhiloxY& y) {
+  uint32_t h, l;
+  mul_wide(y.h ^ x.a, kPhiloxM1, h, l);
+  return philox_rounds<7>(make_uint4(h ^ x.b, l, x.h ^ y.l, x.l), k.k0 + 3 * kPhiloxW0,
+                          k.k1 + 3 * kPhiloxW1);
 }
 
 __device__ __forceinline__ float ex2_approx(float x) {
@@ -76,78 +128,44 @@ __device__ __forceinline__ float cos_approx(float x) {
   return y;
 }
 
-// The Box-Muller angle pi (2 u - 1) of u = uniform_open(w) in one FMA:
-// f = 2 + (w >> 9) 2^-22 (exact, in [2, 4)) and pi (2 u - 1) = pi f - 3 pi +
-// pi 2^-23 in exact arithmetic.
-__device__ __forceinline__ float bm_angle(uint32_t w) {
-  const float f = __uint_as_float(0x40000000u | (w >> 9));
-  return fmaf(3.14159265359f, f, -9.42477758f);  // -3 pi + pi 2^-23, rounded
-}
-
-// Box-Muller on two uniform pairs: (z0,z1) from (w0,w1), (z2,z3) from (w2,w3).
-// z = sqrt(-2 ln u0) * (cos, sin)(pi * (2 u1 - 1)).
-__device__ __forceinline__ float4 normals4(uint4 w) {
-  const float kNeg2Ln2 = -1.38629436112f;  // -2 ln 2: -2 ln u = -2 ln2 * log2 u
-  const float u0 = uniform_open(w.x), u2 = uniform_open(w.z);
-  const float r0 = sqrt_approx(kNeg2Ln2 * lg2_approx(u0));
-  const float r1 = sqrt_approx(kNeg2Ln2 * lg2_approx(u2));
-  const float t0 = bm_angle(w.y);
-  const float t1 = bm_angle(w.w);
-  return make_float4(r0 * cos_approx(t0), r0 * sin_approx(t0), r1 * cos_approx(t1),
-                     r1 * sin_approx(t1));
-}
-
-// normals4 with the two pairs side by side in packed FP32x2 arithmetic: each
-// lane rounds exactly as the scalar operation, so the normals are the same
-// bits; the Monte Carlo kernels, issue-bound, spend fewer instructions on
-// them (the Longstaff-Schwartz forward pass, bound by HBM writes, keeps the
-// scalar form, which measured faster there).
-__device__ __forceinline__ float4 normals4_x2(uint4 w) {
+// Box-Muller on two uniform pairs: (z0,z1) from (w0,w1), (z2,z3) from (w2,w3),
+// z = sqrt(-2 ln u0) * (cos, sin)(pi * (2 u1 - 1)) with u = (2*(w >> 9) + 1) 2^-24.
+// u is exact: 1.m - (1 - 2^-24) is an exact subtraction (Sterbenz), so no
+// integer-to-float conversion is needed; -2 ln u = -2 ln2 * log2 u. The angle is
+// one FMA: f = 2 + (w >> 9) 2^-22 (exact, in [2, 4)) and pi (2 u - 1) = pi f - 3 pi
+// + pi 2^-23 in exact arithmetic. The two pairs run side by side in packed
+// FP32x2 arithmetic: each lane rounds exactly as the scalar operation.
+__device__ __forceinline__ float2 bm_radius(uint32_t wa, uint32_t wb) {
   const float kNeg2Ln2 = -1.38629436112f;
-  const float2 f = __fadd2_rn(make_float2(__uint_as_float(0x3f800000u | (w.x >> 9)),
-                                          __uint_as_float(0x3f800000u | (w.z >> 9))),
-                              make_float2(-0.99999994f, -0.99999994f));  // uniform_open
+  const float2 f = __fadd2_rn(make_float2(__uint_as_float(0x3f800000u | (wa >> 9)),
+                                          __uint_as_float(0x3f800000u | (wb >> 9))),
+                              make_float2(-0.99999994f, -0.99999994f));
   const float2 l = __fmul2_rn(make_float2(kNeg2Ln2, kNeg2Ln2),
                               make_float2(lg2_approx(f.x), lg2_approx(f.y)));
-  const float2 r = make_float2(sqrt_approx(l.x), sqrt_approx(l.y));
-  const float2 t = __ffma2_rn(make_float2(3.14159265359f, 3.14159265359f),
-                              make_float2(__uint_as_float(0x40000000u | (w.y >> 9)),
-                                          __uint_as_float(0x40000000u | (w.w >> 9))),
-                              make_float2(-9.42477758f, -9.42477758f));  // bm_angle
+  return make_float2(sqrt_approx(l.x), sqrt_approx(l.y));
+}
+__device__ __forceinline__ float2 bm_angle(uint32_t wa, uint32_t wb) {
+  return __ffma2_rn(make_float2(3.14159265359f, 3.14159265359f),
+                    make_float2(__uint_as_float(0x40000000u | (wa >> 9)),
+                                __uint_as_float(0x40000000u | (wb >> 9))),
+                    make_float2(-9.42477758f, -9.42477758f));  // -3 pi + pi 2^-23, rounded
+}
+__device__ __forceinline__ float4 normals4_x2(uint4 w) {
+  const float2 r = bm_radius(w.x, w.z), t = bm_angle(w.y, w.w);
   const float2 c = __fmul2_rn(r, make_float2(cos_approx(t.x), cos_approx(t.y)));
   const float2 s = __fmul2_rn(r, make_float2(sin_approx(t.x), sin_approx(t.y)));
   return make_float4(c.x, s.x, c.y, s.y);
 }
 
-// normals4 of two Philox blocks side by side: z[l] holds normal l of block a
-// (.x) and of block b (.y), ready for packed steps of the two paths. The same
-// bits as normals4 of each.
+// normals4_x2 of two Philox blocks: z[l] holds normal l of block a (.x) and of
+// block b (.y), ready for packed steps of the two paths. The same bits.
 __device__ __forceinline__ void normals4_pair(uint4 a, uint4 b, float2 (&z)[4]) {
-  const float kNeg2Ln2 = -1.38629436112f;
-  auto radius = [&](uint32_t wa, uint32_t wb) {
-    const float2 f = __fadd2_rn(make_float2(__uint_as_float(0x3f800000u | (wa >> 9)),
-                                            __uint_as_float(0x3f800000u | (wb >> 9))),
-                                make_float2(-0.99999994f, -0.99999994f));  // uniform_open
-    const float2 l = __fmul2_rn(make_float2(kNeg2Ln2, kNeg2Ln2),
-                                make_float2(lg2_approx(f.x), lg2_approx(f.y)));
-    return make_float2(sqrt_approx(l.x), sqrt_approx(l.y));
-  };
-  auto angle = [&](uint32_t wa, uint32_t wb) {
-    return __ffma2_rn(make_float2(3.14159265359f, 3.14159265359f),
-                      make_float2(__uint_as_float(0x40000000u | (wa >> 9)),
-                                  __uint_as_float(0x40000000u | (wb >> 9))),
-                      make_float2(-9.42477758f, -9.42477758f));  // bm_angle
-  };
-  const float2 r0 = radius(a.x, b.x), t0 = angle(a.y, b.y);
-  const float2 r1 = radius(a.z, b.z), t1 = angle(a.w, b.w);
+  const float2 r0 = bm_radius(a.x, b.x), t0 = bm_angle(a.y, b.y);
+  const float2 r1 = bm_radius(a.z, b.z), t1 = bm_angle(a.w, b.w);
   z[0] = __fmul2_rn(r0, make_float2(cos_approx(t0.x), cos_approx(t0.y)));
   z[1] = __fmul2_rn(r0, make_float2(sin_approx(t0.x), sin_approx(t0.y)));
   z[2] = __fmul2_rn(r1, make_float2(cos_approx(t1.x), cos_approx(t1.y)));
   z[3] = __fmul2_rn(r1, make_float2(sin_approx(t1.x), sin_approx(t1.y)));
-}
-
-__device__ __forceinline__ float lane4(const float4& v, int l) {
-  return l == 0 ? v.x : (l == 1 ? v.y : (l == 2 ? v.z : v.w));
 }
 
 // Kahan-compensated FP32 sum: FP64 is scarce on GB300, so no per-path FP64
