@@ -627,8 +627,8 @@ __device__ void add_chain_warp(const BinomTables& T, double& acc, int& n, int lo
   if (rec && lane == 0) rec->segs = segs;
 }
 
-// Two warps a contract. The first takes the logarithms of u, d and S0 and
-// names the contract of its items; the second walks the comb() accumulator's
+// Two warps a contract. The first takes the logarithms of u, d and S0, names the
+// contract of its items and clears its ticket; the second walks the comb() accumulator's
 // additions from N down through the window. The additions are the same for
 // every term up to where it starts to subtract, so they are walked once; a
 // term then needs one difference.
@@ -651,6 +651,7 @@ __global__ void __launch_bounds__(kPrepBlock) binom_prep_kernel(BinomLaunch L) {
     return;
   }
   for (int k = lane; k < C.items; k += 32) L.item_contract[L.item_start[c] + k] = c;
+  if (lane == 0) L.tickets[c] = 0u;
   if (C.wide) return;
   const __int128 g = lane < 3 ? log2_q96(lane == 0 ? C.u : lane == 1 ? C.d : C.S0) : 0;
   unsigned long long gh = (unsigned long long)(g >> 64), gl = (unsigned long long)g;
@@ -938,20 +939,18 @@ extern "C" int pcf_binom_embar_batch(pcf_ctx* ctx, int n, const pcf_binom_contra
     const size_t h2d = a256(o_start + sizeof(int) * (n + 1));
     const size_t o_part = h2d;
     const size_t o_tick = a256(o_part + sizeof(double) * items);
-    const size_t o_out = a256(o_tick + sizeof(unsigned) * n);
-    const size_t o_prep = a256(o_out + sizeof(double) * n);
+    const size_t o_prep = a256(o_tick + sizeof(unsigned) * n);
     const size_t o_map = a256(o_prep + sizeof(BinomPrep) * n);
     const size_t total = a256(o_map + sizeof(int) * items);
-    st = ctx_ensure(c, total, std::max(h2d, sizeof(double) * n));
+    st = ctx_ensure(c, total, h2d + sizeof(double) * n);
     if (st) return st;
     char* h = (char*)c->h_buf;
     char* d = (char*)c->d_buf;
     memcpy(h + o_cs, cs.data(), sizeof(BinomContract) * n);
     memcpy(h + o_start, start.data(), sizeof(int) * (n + 1));
     st = cuda_status(cudaMemcpyAsync(d, h, h2d, cudaMemcpyHostToDevice, c->stream), "H2D binom");
-    if (!st) st = cuda_status(cudaMemsetAsync(d + o_tick, 0, sizeof(unsigned) * n, c->stream),
-                              "memset binom tickets");
     if (st) return st;
+    double* out = (double*)(h + h2d);  // the kernels write the sums to the pinned buffer
     BinomLaunch L;
     L.cs = (const BinomContract*)(d + o_cs);
     L.item_start = (const int*)(d + o_start);
@@ -959,7 +958,7 @@ extern "C" int pcf_binom_embar_batch(pcf_ctx* ctx, int n, const pcf_binom_contra
     L.total_items = items;
     L.partial = (double*)(d + o_part);
     L.tickets = (unsigned*)(d + o_tick);
-    L.out = (double*)(d + o_out);
+    L.out = out;
     L.mode = mode;
     char* tb = (char*)c->d_logtab;
     L.t.logt = (const double*)tb;
@@ -981,11 +980,9 @@ extern "C" int pcf_binom_embar_batch(pcf_ctx* ctx, int n, const pcf_binom_contra
     c->launches += 1 + (wide < n) + (wide > 0);
     st = cuda_status(cudaGetLastError(), "binom kernel launch");
     if (st) return st;
-    st = cuda_status(cudaMemcpyAsync(h, L.out, sizeof(double) * n, cudaMemcpyDeviceToHost,
-                                     c->stream), "D2H binom");
-    if (!st) st = cuda_status(cudaStreamSynchronize(c->stream), "binom kernel");
+    st = cuda_status(cudaStreamSynchronize(c->stream), "binom kernel");
     if (st) return st;
-    for (int i = 0; i < n; ++i) prices[i] = exp(-ks[i].r * ks[i].T) * ((double*)h)[i];  // :49
+    for (int i = 0; i < n; ++i) prices[i] = exp(-ks[i].r * ks[i].T) * out[i];  // :49
     return PCF_OK;
   });
 }

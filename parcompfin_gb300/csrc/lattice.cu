@@ -510,10 +510,10 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
     const size_t ring_bytes = sizeof(unsigned long long) * kRing * (size_t)strips;
     const size_t o_cnt = a256(o_ring + ring_bytes);
     const size_t cnt_bytes = 256 + a256(sizeof(unsigned) * (size_t)strips);
-    const size_t o_out = o_cnt + cnt_bytes;
-    const size_t o_A = o_out + 256, o_B = a256(o_A + (top < N ? 8 * nodes : 0));
+    const size_t o_out = o_cnt + 128;  // beside the error word: one copy brings both
+    const size_t o_A = o_cnt + cnt_bytes, o_B = a256(o_A + (top < N ? 8 * nodes : 0));
     const size_t total = o_B + (top < N ? 8 * nodes : 0);
-    st = ctx_ensure(c, total, 16 * nodes + 64);
+    st = ctx_ensure(c, total, 16 * nodes + 256);
     if (st) return st;
     char* dv = (char*)c->d_buf;
     double* h = (double*)c->h_buf;
@@ -555,6 +555,7 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
     P.strips = strips;
     P.sms = c->sm_count;
 
+    double root = 0;
     for (;;) {
       st = cuda_status(cudaMemsetAsync(dv + o_cnt, 0, cnt_bytes, c->stream),
                        "memset lattice counters");
@@ -586,19 +587,16 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
                        "lattice strip launch");
       if (st) return st;
       c->launches += 1;
-      st = cuda_status(cudaMemcpyAsync(h, dv + o_out, 8, cudaMemcpyDeviceToHost, c->stream),
+      st = cuda_status(cudaMemcpyAsync(h, dv + o_cnt, 256, cudaMemcpyDeviceToHost, c->stream),
                        "D2H lattice");
-      if (!st)
-        st = cuda_status(cudaMemcpyAsync(h + 1, dv + o_cnt + 64, sizeof(int),
-                                         cudaMemcpyDeviceToHost, c->stream),
-                         "D2H lattice flag");
       if (!st) st = cuda_status(cudaStreamSynchronize(c->stream), "lattice kernel");
       if (st) return st;
-      if (*(const int*)(h + 1)) return set_error(PCF_ETIMEOUT, "lattice grid barrier gave up");
-      if (exact || (h[0] >= 0x1p-700 && std::isfinite(h[0]))) break;
+      if (((const int*)h)[16]) return set_error(PCF_ETIMEOUT, "lattice grid barrier gave up");
+      root = h[16];
+      if (exact || (root >= 0x1p-700 && std::isfinite(root))) break;
       exact = true;  // too small (or not finite) for the three-operation division
     }
-    *price = h[0];
+    *price = root;
     return PCF_OK;
   });
 }

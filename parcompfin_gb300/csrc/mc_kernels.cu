@@ -386,7 +386,7 @@ constexpr int mc_min_blocks() {
 // paths: units_per_item = BS x (paths or quads per thread).
 template <int METHOD, int DMAX, bool CV, int BS>
 __global__ void __launch_bounds__(BS, (mc_min_blocks<METHOD, DMAX, BS>()))
-mc_kernel(McLaunch L) {
+mc_kernel(const __grid_constant__ McLaunch L) {
   __shared__ DF sh[32 * kMoments];
   __shared__ int s_item[2];
   __shared__ int s_c;
@@ -411,7 +411,7 @@ mc_kernel(McLaunch L) {
       item = blockIdx.x;
     }
     if (item >= L.total_items) break;
-    {
+    if (L.contracts) {
       const int t = c + (int)threadIdx.x;
       if (t < L.ncontracts && __ldg(L.item_start + t) <= item &&
           (t + 1 == L.ncontracts || item < __ldg(L.item_start + t + 1)))
@@ -420,8 +420,8 @@ mc_kernel(McLaunch L) {
       const int found = s_c;
       c = found >= 0 ? found : find_contract(L.item_start, L.ncontracts, item);
     }
-    const McContract C = L.contracts[c];
-    const int base = __ldg(L.item_start + c);
+    const McContract C = L.contracts ? L.contracts[c] : L.one;
+    const int base = L.contracts ? __ldg(L.item_start + c) : 0;
     const int j = item - base;
     Moments<CV> mo;
     if (METHOD == MC_EUR) {
@@ -540,7 +540,7 @@ constexpr size_t tc_basket_smem() {  // l0, v | L_hi, L_lo | 2 x (Z_hi, Z_lo) ch
 }
 
 template <int DMAX, bool CV>
-__global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(McLaunch L) {
+__global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(const __grid_constant__ McLaunch L) {
   static_assert(DMAX == 32 || DMAX == 64, "tensor-core baskets: 17..64 assets");
   extern __shared__ __align__(128) float s_tc[];
   __shared__ DF sh[32 * kMoments];
@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(McLaunch L) {
       item = blockIdx.x;
     }
     if (item >= L.total_items) break;
-    {
+    if (L.contracts) {
       const int t = c + tid;
       if (t < L.ncontracts && __ldg(L.item_start + t) <= item &&
           (t + 1 == L.ncontracts || item < __ldg(L.item_start + t + 1)))
@@ -603,8 +603,8 @@ __global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(McLaunch L) {
       const int found = s_c;
       c = found >= 0 ? found : find_contract(L.item_start, L.ncontracts, item);
     }
-    const McContract C = L.contracts[c];
-    const int base = __ldg(L.item_start + c);
+    const McContract C = L.contracts ? L.contracts[c] : L.one;
+    const int base = L.contracts ? __ldg(L.item_start + c) : 0;
     const int j = item - base;
     const int d = C.M;
     if (loaded != c) {

@@ -24,6 +24,7 @@ struct pcf_ctx {
   size_t d_cap = 0;
   void* h_buf = nullptr;  // pinned staging
   size_t h_cap = 0;
+  unsigned* d_ticket = nullptr;  // 0 between calls: the single-contract launches' ticket
   // Longstaff-Schwartz path matrix and per-path state, kept resident.
   void* d_paths = nullptr;
   size_t paths_cap = 0;

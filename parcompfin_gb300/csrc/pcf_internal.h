@@ -38,7 +38,7 @@ struct McContract {
 // Basket factor block (device): per asset log2(S0_a) + (r - s_a^2/2) T log2e,
 // s_a * ts * log2e, then the d x d lower Cholesky factor, row-major, FP32.
 struct McLaunch {
-  const McContract* contracts;
+  const McContract* contracts;  // NULL: one contract, `one`, passed with the launch
   const int* item_start;   // exclusive prefix of items per contract, size C+1
   const float* basket_data;
   int ncontracts;
@@ -49,6 +49,7 @@ struct McLaunch {
   double* out;             // ncontracts * kMoments
   int persistent;
   int cv;                  // accumulate the control-variate sums (else they are 0)
+  McContract one;
 };
 
 enum McMethod { MC_EUR = 0, MC_ASIA = 1, MC_BASKET = 2 };
