@@ -881,7 +881,7 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
   }
   DF v[kMoments] = {df_of(sy), df_of(syy), df_of(sg), df_of(sgg), df_of(syg)};
   DF tot[kMoments];
-  block_sum_df<kMoments>(v, X.sh, tot);
+  block_sum_df<kMoments, BS / 32>(v, X.sh, tot);
   if (CLUSTER) {
     if (threadIdx.x == 0)
       for (int q = 0; q < kMoments; ++q) X.fin[q] = tot[q];
@@ -1076,7 +1076,7 @@ __global__ void __launch_bounds__(kLsmBlock, 1) lsm_stream_kernel(LsmParams P) {
   }
   DF v[kMoments] = {df_of(sy), df_of(syy), df_of(sg), df_of(sgg), df_of(syg)};
   DF tot[kMoments];
-  block_sum_df<kMoments>(v, X.sh, tot);
+  block_sum_df<kMoments, BS / 32>(v, X.sh, tot);
   grid_finalize_df<kMoments>(tot, (float2*)P.fpartial, P.ticket, P.out, P.nblocks, b);
 }
 

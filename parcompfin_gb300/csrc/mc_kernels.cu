@@ -54,6 +54,23 @@ struct Moments {
   }
 };
 
+// A block's totals of its threads' moments; without the control variate its
+// three sums are zero.
+template <bool CV, int NW>
+__device__ __forceinline__ void item_totals(const Moments<CV>& mo, DF* sh, DF (&tot)[kMoments]) {
+  if (CV) {
+    const DF v[kMoments] = {df_of(mo.y), df_of(mo.yy), df_of(mo.g), df_of(mo.gg), df_of(mo.yg)};
+    block_sum_df<kMoments, NW>(v, sh, tot);
+  } else {
+    const DF v[2] = {df_of(mo.y), df_of(mo.yy)};
+    DF t[2];
+    block_sum_df<2, NW>(v, sh, t);
+    tot[0] = t[0];
+    tot[1] = t[1];
+    tot[2] = tot[3] = tot[4] = DF{0.f, 0.f};
+  }
+}
+
 __device__ __forceinline__ float payoff(const McContract& C, float S) {
   return fmaxf(fmaf(C.pf, S, C.nK), 0.f);  // max(pf (S - K), 0)
 }
@@ -452,9 +469,8 @@ mc_kernel(const __grid_constant__ McLaunch L) {
       }
       basket_item<DMAX, CV, BS>(C, j, s_fb, mo);
     }
-    DF v[kMoments] = {df_of(mo.y), df_of(mo.yy), df_of(mo.g), df_of(mo.gg), df_of(mo.yg)};
     DF tot[kMoments];
-    block_sum_df<kMoments>(v, sh, tot);
+    item_totals<CV, BS / 32>(mo, sh, tot);
     grid_finalize_df<kMoments>(tot, (float2*)L.partial + (size_t)base * kMoments, L.tickets + c,
                                L.out + (size_t)c * kMoments, C.items, j);
     if (threadIdx.x == 0) s_c = -1;  // every thread read s_c before block_sum_df's barriers
@@ -694,9 +710,8 @@ __global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(const __grid_
         mo.add(Y, G);
       }
     }
-    DF v[kMoments] = {df_of(mo.y), df_of(mo.yy), df_of(mo.g), df_of(mo.gg), df_of(mo.yg)};
     DF tot[kMoments];
-    block_sum_df<kMoments>(v, sh, tot);
+    item_totals<CV, kTcBlock / 32>(mo, sh, tot);
     grid_finalize_df<kMoments>(tot, (float2*)L.partial + (size_t)base * kMoments, L.tickets + c,
                                L.out + (size_t)c * kMoments, C.items, j);
     if (tid == 0) s_c = -1;
@@ -875,9 +890,8 @@ __global__ void __launch_bounds__(kBlock) mc_eur_noalloc_kernel(McContract C,
   const int j = blockIdx.x;
   Moments<true> mo;
   eur_item<true, kBlock>(C, j, mo);
-  DF v[kMoments] = {df_of(mo.y), df_of(mo.yy), df_of(mo.g), df_of(mo.gg), df_of(mo.yg)};
   DF tot[kMoments];
-  block_sum_df<kMoments>(v, sh, tot);
+  item_totals<true, kBlock / 32>(mo, sh, tot);
   grid_finalize_df<kMoments>(tot, partial, ticket, out, C.items, j);
 }
 

@@ -249,23 +249,50 @@ __device__ __forceinline__ DF warp_sum_df(DF v) {
   return v;
 }
 
-// Sums K double-floats over the block; thread 0 gets the totals. `sh` must
-// hold 32*K DFs. Deterministic for a fixed block size.
-template <int K>
-__device__ __forceinline__ void block_sum_df(DF (&v)[K], DF* sh, DF (&out)[K]) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+// Sums K <= 8 double-floats over a block of NW warps (a power of two); every
+// lane of warp 0 gets the totals. `sh` must hold NW*K DFs. Deterministic: a
+// butterfly over the lanes, then one over the warps. Both are reduce-scatters:
+// a step halves the sums a lane still carries (9 shuffled additions a warp for
+// five sums instead of 25, 6 instead of 25 over eight warps). A double-float
+// addition gives the same bits in either order of its operands, so the totals
+// are those of a full butterfly. The sums of an item cost as much as 20 path
+// quads before.
+template <int K, int NW>
+__device__ __forceinline__ void block_sum_df(const DF (&v)[K], DF* sh, DF (&out)[K]) {
+  static_assert(K <= 8 && NW >= 4 && NW <= 32 && (NW & (NW - 1)) == 0, "block shape");
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+  const DF zero{0.f, 0.f};
+  auto pick = [](bool c, DF x, DF y) { return DF{c ? x.hi : y.hi, c ? x.lo : y.lo}; };
+  DF w4[4], w2[2];
 #pragma unroll
-  for (int k = 0; k < K; ++k) v[k] = warp_sum_df(v[k]);
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) sh[wid * K + k] = v[k];
+  for (int i = 0; i < 4; ++i) {  // lanes with bit 4 keep sums 4..7, the others 0..3
+    const DF lo = i < K ? v[i] : zero, hi = i + 4 < K ? v[i + 4] : zero;
+    if (i < K) w4[i] = df_add(pick(b4, hi, lo), shfl_xor_df(pick(b4, lo, hi), 16));
+    else w4[i] = zero;
   }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (i < K) w2[i] = df_add(pick(b3, w4[i + 2], w4[i]), shfl_xor_df(pick(b3, w4[i], w4[i + 2]), 8));
+    else w2[i] = zero;
+  }
+  DF x = df_add(pick(b2, w2[1], w2[0]), shfl_xor_df(pick(b2, w2[0], w2[1]), 4));
+  x = df_add(x, shfl_xor_df(x, 2));
+  x = df_add(x, shfl_xor_df(x, 1));
+  const int q = lane >> 2;  // the sum this lane ended with
+  if ((lane & 3) == 0 && q < K) sh[wid * K + q] = x;
   __syncthreads();
   if (wid == 0) {
+    constexpr int kPer = 32 / NW;  // sums a pass, one per NW lanes
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      DF x = lane < nw ? sh[lane * K + k] : DF{0.f, 0.f};
-      out[k] = warp_sum_df(x);
+    for (int k0 = 0; k0 < K; k0 += kPer) {
+      const int k = k0 + lane / NW;
+      DF y = k < K ? sh[(lane & (NW - 1)) * K + k] : zero;
+#pragma unroll
+      for (int o = NW / 2; o > 0; o >>= 1) y = df_add(y, shfl_xor_df(y, o));
+#pragma unroll
+      for (int i = 0; i < kPer; ++i)
+        if (k0 + i < K) out[k0 + i] = shfl_df(y, i * NW);
     }
   }
   __syncthreads();
