@@ -26,6 +26,8 @@ raw moment sums).
 from __future__ import annotations
 
 import ctypes as C
+import struct
+from itertools import chain
 
 from . import _lib
 
@@ -229,13 +231,42 @@ def binom_embar(S0, E, r, sigma, T, N, payoff_fun, *, mode="reference", ctx=None
     return out.value
 
 
+_PAYOFF_CODES = {1: 1, -1: -1, "call": 1, "put": -1}
+
+
+def _pack_binom(cs):
+    """The contracts as a ctypes array, packed by one call: seven attribute
+    stores a contract took 0.7 of the 1.2 ms of a 1024-contract call."""
+    n = len(cs)
+    try:
+        if set(map(len, cs)) != {7}:
+            raise TypeError
+        flat = list(chain.from_iterable(cs))
+        codes = list(map(_PAYOFF_CODES.__getitem__, flat[6::7]))
+    except (TypeError, KeyError):  # rows without a length, payoffs of other types
+        rows = [tuple(c) for c in cs]
+        if any(len(row) != 7 for row in rows):
+            raise ValueError("a contract is (S0, E, r, sigma, T, N, payoff_fun)") from None
+        flat = list(chain.from_iterable(rows))
+        codes = [payoff_code(p) for p in flat[6::7]]
+    flat[6::7] = codes
+    form = struct.Struct("5d2i" * n)
+    try:
+        buf = form.pack(*flat)
+    except struct.error:  # N is not a plain int, or exceeds 32 bits (a C int drops the rest)
+        flat[5::7] = [C.c_int32(int(x)).value for x in flat[5::7]]
+        try:
+            buf = form.pack(*flat)
+        except struct.error as e:
+            raise TypeError(str(e)) from None
+    return (_lib.BinomContract * n).from_buffer_copy(buf)
+
+
 def binom_embar_batch(contracts, *, mode="reference", ctx=None) -> list:
     """contracts: iterable of (S0, E, r, sigma, T, N, payoff_fun); one launch."""
     lib = _lib.load()
     cs = list(contracts)
-    arr = (_lib.BinomContract * len(cs))()
-    for k, (S0, E, r, sigma, T, N, pf) in enumerate(cs):
-        arr[k] = _lib.BinomContract(S0, E, r, sigma, T, int(N), payoff_code(pf))
+    arr = _pack_binom(cs) if cs else (_lib.BinomContract * 0)()
     out = (C.c_double * len(cs))()
     _lib.check(lib.pcf_binom_embar_batch(_h(ctx), len(cs), arr, BINOM_MODES.get(mode, mode), out))
     return list(out)

@@ -102,3 +102,25 @@ def test_no_device_fails_loudly(pcf_lib):
     from parcompfin_gb300 import PcfError, mc_eur
     with pytest.raises(PcfError):
         mc_eur(100, 100, .05, .2, 1, 1000, "call")
+
+
+def test_binom_batch_packing_matches_field_by_field():
+    """The columns that binom_embar_batch packs are the fields a contract-by-
+    contract assignment gives, for the argument types it accepts; what is not a
+    contract is refused."""
+    np = pytest.importorskip("numpy")
+    from parcompfin_gb300 import _lib, api, workloads
+    rows = workloads.binom_book(37) + [
+        [100, np.float64(110), .02, .75, 1, np.int64(100), "put"],
+        (100.0, 110, .02, .75, 1.0, 7.9, 1.0), (1, 2, 3, .4, 5, 2**32 + 6, True)]
+    want = (_lib.BinomContract * len(rows))()
+    for k, (S0, E, r, sigma, T, N, pf) in enumerate(rows):
+        want[k] = _lib.BinomContract(S0, E, r, sigma, T, int(N), api.payoff_code(pf))
+    assert bytes(api._pack_binom(rows)) == bytes(want)
+    assert bytes(api._pack_binom([iter(r) for r in rows])) == bytes(want)
+    for bad in ([(1, 2, 3, 4, 5, 6)], [(1, 2, 3, 4, 5, 6, "x")], [(1, 2, 3, 4, 5, 6, 0)],
+                [(1, 2, 3, 4, 5, 6, 7, 8), (1, 2, 3, 4, 5, 6)]):
+        with pytest.raises(ValueError):
+            api._pack_binom(bad)
+    with pytest.raises(TypeError):
+        api._pack_binom([(1, "2", 3, 4, 5, 6, "put")])
