@@ -481,22 +481,34 @@ mc_kernel(const __grid_constant__ McLaunch L) {
 // ---- baskets of more than 16 assets: the L z product on the tensor cores ----
 //
 // A tile is 128 paths (one per thread); the product X = Z L^T of a tile runs
-// on the tensor cores, K (the assets) in chunks of 8. For each chunk every
-// thread draws its path's next 8 normals and stores them, split into two
-// TF32 parts z = z_hi + z_lo, as row `tid` of a 128 x 8 K-major chunk in
-// shared memory (double-buffered); one thread then issues three
+// on the tensor cores, K (the assets) in chunks of 16. For each chunk every
+// thread draws its path's next 16 normals into registers and then stores them,
+// split into two TF32 parts z = z_hi + z_lo, as row `tid` of a 128 x 16 K-major
+// chunk in shared memory; one thread then issues, for each 8 assets, three
 // tcgen05.mma kind::tf32 (M = 128, N = d rounded up to 16, K = 8)
 // accumulating X += Z_hi L_hi^T + Z_lo L_hi^T + Z_hi L_lo^T in tensor memory
-// and commits them to the chunk buffer's mbarrier, so drawing chunk c + 1
-// overlaps the MMAs of chunk c. The dropped Z_lo L_lo^T term is below 2^-22
-// of the product: X carries FP32-level accuracy. The factor is staged once
-// per contract, split the same way. After the last chunk each warp reads its
-// 32 rows of X (tcgen05.ld 32x32b) and finishes its paths on the CUDA cores.
-// Shared-memory operands use the canonical K-major layout without swizzle:
-// 8-row x 16-byte core matrices, adjacent along K 128 bytes apart (leading
-// offset) and along M/N (K/4) x 128 bytes apart (stride offset). A chunk
-// buffer is 16 KB, so four CTAs share an SM.
+// and commits them to the chunk's mbarrier. The next chunk's draws need no
+// shared memory, so they run while those MMAs do: one buffer is enough, and
+// the wait before the stores finds it free. The dropped Z_lo L_lo^T term is
+// below 2^-22 of the product: X carries FP32-level accuracy. The factor is
+// staged once per contract, split the same way. After the last chunk each warp
+// reads its 32 rows of X (tcgen05.ld 32x32b) and finishes its paths on the
+// CUDA cores. Shared-memory operands use the canonical K-major layout without
+// swizzle: 8-row x 16-byte core matrices, adjacent along K 128 bytes apart
+// (leading offset) and along M/N (K/4) x 128 bytes apart (stride offset).
+//
+// What bounds it is issue: 0.6 of the slots busy, no pipe above 0.46 (ALU;
+// tensor pipe 0.18), the rest waits of few warps on one another. Baskets of 4,
+// 16 and 64 assets, 2^22 paths each, of which this kernel was 548 us: 709 us
+// with two 8-asset buffers and four CTAs an SM; 652 with one (five CTAs fit);
+// 625 with TF32 rounding on the integer pipe instead of cvt.rna.tf32; 584 with
+// the sums over the assets in unpredicated groups of eight; 572 with these in
+// packed FMAs; 564 with 16-asset chunks (half the barriers, four draws in
+// flight; four CTAs of 64 assets again, seven of 32); 550 without the zero fill
+// of normals beyond d. Two tiles a CTA around one factor (24 warps an SM instead
+// of 16) took 2 us off the 564, but the mixed stream was 1 % slower.
 constexpr int kTcBlock = 128;
+constexpr int kTcK = 16;  // assets in a chunk
 
 __device__ __forceinline__ uint32_t kmajor_off(int row, int k, int ktot) {
   return (uint32_t)((row >> 3) * (ktot >> 2) * 128 + (k >> 2) * 128 + (row & 7) * 16 +
@@ -509,10 +521,10 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
          ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
 }
 
+// x rounded to TF32 (10 stored mantissa bits), ties away from zero: what
+// cvt.rna.tf32 does to a finite x far from overflow, on the integer pipe.
 __device__ __forceinline__ float tf32_round(float x) {
-  uint32_t r;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-  return __uint_as_float(r);
+  return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
 }
 
 __device__ __forceinline__ void umma_tf32(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc,
@@ -548,27 +560,36 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-constexpr int kTcChunk = kTcBlock * 8;  // floats in one 128 x 8 chunk
+constexpr int kTcChunk = kTcBlock * kTcK;  // floats in one 128 x 16 chunk
 
 template <int DMAX>
-constexpr size_t tc_basket_smem() {  // l0, v | L_hi, L_lo | 2 x (Z_hi, Z_lo) chunks (floats)
-  return (size_t)(2 * DMAX + 2 * DMAX * DMAX + 4 * kTcChunk) * sizeof(float);
+constexpr size_t tc_basket_smem() {  // l0, v | L_hi, L_lo | a chunk's Z_hi, Z_lo (floats)
+  return (size_t)(2 * DMAX + 2 * DMAX * DMAX + 2 * kTcChunk) * sizeof(float);
+}
+
+// CTAs on an SM: what shared memory holds (48.5 or 24.3 KB a CTA) and, for 32
+// assets, 72 registers a thread.
+template <int DMAX>
+constexpr int tc_ctas() {
+  return DMAX == 32 ? 7 : 4;
 }
 
 template <int DMAX, bool CV>
-__global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(const __grid_constant__ McLaunch L) {
+__global__ void __launch_bounds__(kTcBlock, (tc_ctas<DMAX>()))
+mc_basket_tc_kernel(const __grid_constant__ McLaunch L) {
   static_assert(DMAX == 32 || DMAX == 64, "tensor-core baskets: 17..64 assets");
   extern __shared__ __align__(128) float s_tc[];
   __shared__ DF sh[32 * kMoments];
   __shared__ int s_item[2];
   __shared__ int s_c;
-  __shared__ __align__(8) uint64_t mbar[2];
+  __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t s_tmem;
   float* l0 = s_tc;
   float* vol = s_tc + DMAX;
   float* Lhi = s_tc + 2 * DMAX;
   float* Llo = Lhi + DMAX * DMAX;
-  float* Zc = Llo + DMAX * DMAX;  // buffer b: Z_hi at Zc + 2 b chunk, Z_lo next to it
+  float* zh = Llo + DMAX * DMAX;
+  float* zl = zh + kTcChunk;
   const int tid = threadIdx.x, warp = tid >> 5;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -578,8 +599,7 @@ __global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(const __grid_
   }
   if (tid == 0) {
     s_c = -1;
-    mbar_init(&mbar[0], 1);
-    mbar_init(&mbar[1], 1);
+    mbar_init(&mbar, 1);
     fence_mbar_init();
     if (L.persistent) s_item[0] = (int)atomicAdd(L.queue, 1u);
   }
@@ -589,15 +609,15 @@ __global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(const __grid_
   const uint32_t tmem = s_tmem;
   const uint32_t row_tmem = tmem + ((uint32_t)(warp * 32) << 16);
   const uint32_t sbo_l = (DMAX / 4) * 128;
-  const uint32_t z_off = kmajor_off(tid, 0, 8) >> 2;  // this thread's row in a chunk
-  uint32_t phase = 0;   // bit b: parity of the next wait on mbar[b]
-  uint32_t pending = 0; // bit b: a commit on mbar[b] not yet waited
+  const uint32_t z_off = kmajor_off(tid, 0, kTcK) >> 2;  // this thread's row in a chunk
+  uint32_t phase = 0;    // parity of the next wait on mbar
+  bool pending = false;  // a commit on mbar not yet waited for
   bool failed = false;
-  auto wait_buf = [&](int b) {
-    if (!((pending >> b) & 1u)) return;
-    if (!mbar_poll(&mbar[b], (phase >> b) & 1u, 1u << 24)) failed = true;
-    phase ^= 1u << b;
-    pending &= ~(1u << b);
+  auto wait_mma = [&]() {
+    if (!pending) return;
+    if (!mbar_poll(&mbar, phase, 1u << 24)) failed = true;
+    phase ^= 1u;
+    pending = false;
   };
   int c = 0, loaded = -1;
   for (int iter = 0;; ++iter) {
@@ -641,7 +661,7 @@ __global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(const __grid_
       }
       loaded = c;
     }
-    const int nchunks = (d + 7) >> 3, np = (d + 15) & ~15;
+    const int np = (d + 15) & ~15;
     // D f32, A and B tf32, both K-major; N >> 3 at bit 17, M >> 4 at bit 24.
     const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(np >> 3) << 17) |
                            ((uint32_t)(kTcBlock >> 4) << 24);
@@ -649,42 +669,62 @@ __global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(const __grid_
     Moments<CV> mo;
     for (int tile = 0; tile < C.units_per_item / kTcBlock; ++tile) {
       const long long n = (long long)j * C.units_per_item + (long long)tile * kTcBlock + tid;
-      for (int ch = 0; ch < nchunks; ++ch) {
-        const int b = ch & 1;
-        wait_buf(b);  // the MMAs that read buffer b two chunks ago are done
-        float* zh = Zc + 2 * b * kTcChunk;
-        float* zl = zh + kTcChunk;
+      const PhiloxX px = philox_x(key, (uint64_t)(C.x0 + n));
+#pragma unroll 1
+      for (int k0 = 0; k0 < d; k0 += kTcK) {
+        // Eight assets at a time; normals beyond d meet zero columns of L, and
+        // an eight that starts beyond d is neither drawn nor multiplied.
+        float z[kTcK];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int k4 = 2 * ch + h;
-          float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (4 * k4 < d) z = normals4_x2(draw_words(key, (uint64_t)(C.x0 + n), (uint32_t)k4));
-          const float4 hi = make_float4(tf32_round(z.x), tf32_round(z.y), tf32_round(z.z),
-                                        tf32_round(z.w));
-          const float4 lo = make_float4(tf32_round(z.x - hi.x), tf32_round(z.y - hi.y),
-                                        tf32_round(z.z - hi.z), tf32_round(z.w - hi.w));
-          *reinterpret_cast<float4*>(zh + z_off + 32 * h) = hi;  // +128 bytes: next core matrix
-          *reinterpret_cast<float4*>(zl + z_off + 32 * h) = lo;
+        for (int h = 0; h < kTcK / 8; ++h) {
+          if (k0 + 8 * h < d) {
+            const uint32_t y = (uint32_t)(k0 / 4 + 2 * h);
+            float2 zz[4];
+            normals4_pair(draw_words(key, px, philox_y(key, y)),
+                          draw_words(key, px, philox_y(key, y + 1)), zz);
+#pragma unroll
+            for (int l = 0; l < 4; ++l) z[8 * h + l] = zz[l].x, z[8 * h + 4 + l] = zz[l].y;
+          }
+        }
+        wait_mma();  // the MMAs that read the previous chunk are done
+#pragma unroll
+        for (int h = 0; h < kTcK / 4; ++h) {
+          if (k0 + 4 * (h & ~1) < d) {
+            const float4 hi = make_float4(tf32_round(z[4 * h]), tf32_round(z[4 * h + 1]),
+                                          tf32_round(z[4 * h + 2]), tf32_round(z[4 * h + 3]));
+            const float4 lo =
+                make_float4(tf32_round(z[4 * h] - hi.x), tf32_round(z[4 * h + 1] - hi.y),
+                            tf32_round(z[4 * h + 2] - hi.z), tf32_round(z[4 * h + 3] - hi.w));
+            *reinterpret_cast<float4*>(zh + z_off + 32 * h) = hi;  // +128 bytes: next core matrix
+            *reinterpret_cast<float4*>(zl + z_off + 32 * h) = lo;
+          }
         }
         // The chunk (and a newly staged factor) is visible to the tensor core;
-        // at ch = 0 every thread has also read the previous tile's X.
+        // at k0 = 0 every thread has also read the previous tile's X.
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (tid == 0) {
-          const uint32_t ah = smem_u32(zh), al = smem_u32(zl);
-          const uint32_t bo = (uint32_t)ch * 256;  // chunk ch: two core matrices along K
-          const uint32_t bh = smem_u32(Lhi) + bo, bl = smem_u32(Llo) + bo;
-          umma_tf32(tmem, umma_desc(ah, 128, 256), umma_desc(bh, 128, sbo_l), idesc, ch > 0);
-          umma_tf32(tmem, umma_desc(al, 128, 256), umma_desc(bh, 128, sbo_l), idesc, 1);
-          umma_tf32(tmem, umma_desc(ah, 128, 256), umma_desc(bl, 128, sbo_l), idesc, 1);
-          umma_commit(&mbar[b]);
+#pragma unroll
+          for (int h = 0; h < kTcK / 8; ++h) {
+            if (k0 + 8 * h < d) {
+              const uint32_t ao = (uint32_t)h * 256;  // two core matrices along K
+              const uint32_t bo = (uint32_t)(k0 + 8 * h) * 32;
+              const uint64_t ah = umma_desc(smem_u32(zh) + ao, 128, kTcK * 32);
+              const uint64_t al = umma_desc(smem_u32(zl) + ao, 128, kTcK * 32);
+              const uint64_t bh = umma_desc(smem_u32(Lhi) + bo, 128, sbo_l);
+              const uint64_t bl = umma_desc(smem_u32(Llo) + bo, 128, sbo_l);
+              umma_tf32(tmem, ah, bh, idesc, k0 + h > 0);
+              umma_tf32(tmem, al, bh, idesc, 1);
+              umma_tf32(tmem, ah, bl, idesc, 1);
+            }
+          }
+          umma_commit(&mbar);
         }
-        pending |= 1u << b;
+        pending = true;
       }
-      wait_buf(0);
-      wait_buf(1);
+      wait_mma();
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       float bsk = 0.f, geo = 0.f;
 #pragma unroll
@@ -692,12 +732,36 @@ __global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(const __grid_
         if (32 * half < np) {
           float x[32];
           tmem_ld32(row_tmem + 32 * half, x);
+          // Full groups of eight assets without a test for each.
 #pragma unroll
-          for (int a = 0; a < 32; ++a) {
-            if (32 * half + a < d) {
-              const float l2 = fmaf(vol[32 * half + a], x[a], l0[32 * half + a]);
-              bsk += ex2_approx(l2);
-              geo += l2;
+          for (int g = 0; g < 4; ++g) {
+            const int a0 = 32 * half + 8 * g;
+            float2 l2[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+              l2[p] = __ffma2_rn(*reinterpret_cast<const float2*>(vol + a0 + 2 * p),
+                                 make_float2(x[8 * g + 2 * p], x[8 * g + 2 * p + 1]),
+                                 *reinterpret_cast<const float2*>(l0 + a0 + 2 * p));
+            if (a0 + 8 <= d) {
+#pragma unroll
+              for (int p = 0; p < 4; ++p) {
+                bsk += ex2_approx(l2[p].x);
+                geo += l2[p].x;
+                bsk += ex2_approx(l2[p].y);
+                geo += l2[p].y;
+              }
+            } else {
+#pragma unroll
+              for (int p = 0; p < 4; ++p) {
+                if (a0 + 2 * p < d) {
+                  bsk += ex2_approx(l2[p].x);
+                  geo += l2[p].x;
+                }
+                if (a0 + 2 * p + 1 < d) {
+                  bsk += ex2_approx(l2[p].y);
+                  geo += l2[p].y;
+                }
+              }
             }
           }
         }
@@ -728,7 +792,7 @@ __global__ void __launch_bounds__(kTcBlock, 4) mc_basket_tc_kernel(const __grid_
 }
 
 // Dynamic shared memory above 48 KB and the largest shared-memory carveout,
-// so that four CTAs share an SM. Function attributes belong to the current
+// so that tc_ctas() share an SM. Function attributes belong to the current
 // device, so they are set on every launch (two host calls, no device work).
 template <int DMAX, bool CV>
 void tc_setup() {
@@ -746,9 +810,9 @@ cudaError_t launch_tc(const McLaunch& L, int grid, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// CTAs per SM: the launch bound (4) caps the registers; shared memory
+// CTAs per SM: the launch bound caps the registers; shared memory
 // decides the rest. (The occupancy query reports one CTA per SM for this
-// kernel, which leaves three quarters of each SM idle; a persistent launch
+// kernel, which leaves most of each SM idle; a persistent launch
 // of more CTAs than fit would only queue them.)
 template <int DMAX>
 int tc_max_active(void) {
@@ -766,7 +830,7 @@ int tc_max_active(void) {
     return 1;
   }
   const size_t per = tc_basket_smem<DMAX>() + fa.sharedSizeBytes + (size_t)reserved;
-  return std::max(1, std::min(4, (int)((size_t)smem_sm / per)));
+  return std::max(1, std::min(tc_ctas<DMAX>(), (int)((size_t)smem_sm / per)));
 }
 
 constexpr size_t basket_smem(int dmax) { return (size_t)(2 + dmax) * dmax * sizeof(float); }

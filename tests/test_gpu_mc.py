@@ -182,6 +182,28 @@ def test_basket_matches_fp64_twin(orc, ctx, d):
         assert rel(res.sums[k], s[k]) < DET_REL, (k, res.sums[k], s[k])
 
 
+# The tensor-core kernel's edges: the last chunk of 16 assets with one asset, a
+# whole eight, an eight and one, or all but one; path counts around its tile of
+# 128 and its item of 1024. The same twin and bound as above.
+@pytest.mark.parametrize("d,N", [(25, 1), (31, 127), (40, 128), (41, 129), (49, 1023), (52, 1025),
+                                 (56, 4097), (57, 3000), (63, 2049)])
+def test_basket_tensor_edges_match_fp64_twin(orc, ctx, d, N):
+    from parcompfin_gb300 import mc_basket_result
+    import random
+    rng = random.Random(d)
+    S0 = [100.0 + rng.uniform(-5, 5) for _ in range(d)]
+    sig = [rng.uniform(.15, .35) for _ in range(d)]
+    corr = [1.0 if i == j else .3 for i in range(d) for j in range(d)]
+    res = mc_basket_result(S0, sig, corr, .03, 1.0, 90.0, N, 1, scale_by_sqrt_T=True, seed=5,
+                           use_cv=True, ctx=ctx)
+    s = (C.c_double * 5)()
+    A = C.c_double * d
+    orc.twin_mc_basket(d, A(*S0), A(*sig), (C.c_double * (d * d))(*_chol(corr, d)), .03, 1.0, 1.0,
+                       90.0, N, 1, 5, 0, s)
+    for k in range(5):
+        assert rel(res.sums[k], s[k]) < DET_REL, (k, res.sums[k], s[k])
+
+
 def test_basket_reference_article_values(ctx):
     """results/results_mc_eur_multi.csv:19 -- the reference prices the d=4,
     rho=.5 basket (S0=K=100, r=.1, sigma=.2, T=1) at 11.9205 with 1e8 paths."""
