@@ -51,9 +51,9 @@ __device__ __forceinline__ uint4 philox_rounds(uint4 c, uint32_t k0, uint32_t k1
   return c;
 }
 
-// One block. The basket kernels and the Longstaff-Schwartz forward pass, whose
-// registers are full, measured 1 to 5 % slower with mul_wide's register pairs
-// (basket book 720 -> 758 us), so the compiler chooses here.
+// One block. The Longstaff-Schwartz forward pass, whose registers are full,
+// measured 1 % slower with mul_wide's register pairs (64-put batch 527 -> 533
+// us), so the compiler chooses here.
 __device__ __forceinline__ uint4 draw_words(const RngKey& k, uint64_t x, uint32_t y) {
   uint4 c = make_uint4((uint32_t)x, y, k.stream, (k.tag << 16) | ((uint32_t)(x >> 32) & 0xffffu));
   uint32_t k0 = k.k0, k1 = k.k1;
