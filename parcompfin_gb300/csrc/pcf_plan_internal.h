@@ -17,6 +17,7 @@ struct Group {  // one persistent Monte Carlo launch
   std::vector<int> start;     // item prefix, size C+1
   McLaunch L{};
   int grid = 0;
+  double draws = 0;           // normals its contracts draw
 };
 
 }  // namespace pcf
@@ -47,9 +48,16 @@ struct pcf_plan {
   // CUDA graph replay: the second launch captures the launch sequence, later
   // launches replay it. graph_mode 0 never captures.
   // Fork/join: the LSM cluster launches run on `side`, concurrently with the
-  // Monte Carlo groups on `stream`, so each fills the other's tail.
+  // Monte Carlo groups on `stream`, so each fills the other's tail; the groups
+  // of a plan of several (that owns its memory) take turns on `stream` and the
+  // lanes for the same reason.
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  struct Lane {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t join = nullptr;
+  };
+  std::vector<Lane> lanes;
   int graph_mode = 1;
   long long launches_done = 0;
   bool graph_failed = false;

@@ -115,6 +115,25 @@ def test_plan_replay_is_deterministic(ctx):
         assert list(a.sums) == list(b.sums)
 
 
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("ds", [(3, 64), (64, 3), (2, 6, 12, 20, 28, 50), (40,)])
+def test_plan_groups_on_several_streams(ctx, ds, graph):
+    """A plan's groups run on up to three streams, the largest first: every
+    launch, direct or replayed, gives each contract the sums it has alone."""
+    import parcompfin_gb300 as pcf
+    reqs = [pcf.request("basket", 100, 95, .03, .25, 1.0, 20000 + 128 * d, "call", assets=d, rho=.3,
+                        use_cv=True, seed=4, stream=d) for d in ds]
+    reqs += [pcf.request("eur", 100, 100, .05, .2, 1.0, 300001, "call", seed=4, stream=100),
+             pcf.request("asia", 100, 100, .05, .2, 1.0, 50003, "call", M=30, seed=4, stream=101),
+             pcf.request("amer", 100, 100, .05, .3, 1.0, 1 << 14, "put", M=20, seed=4, stream=102)]
+    for sel in (reqs[:len(ds)], reqs):
+        want = [list(pcf.price_batch([q], ctx=ctx)[0].sums) for q in sel]
+        with pcf.Plan(sel, ctx=ctx, graph=graph) as plan:
+            for _ in range(4):
+                plan.launch()
+                assert [list(r.sums) for r in plan.results()] == want
+
+
 def test_batch_rejects_bad_requests(ctx):
     import parcompfin_gb300 as pcf
     with pytest.raises(ValueError, match="divisible by 2"):
