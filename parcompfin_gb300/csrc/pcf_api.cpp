@@ -325,6 +325,11 @@ int pcf_ctx_destroy(pcf_ctx* c) {
     ctx_release_extras(c);
     if (c->d_buf) cudaFree(c->d_buf);
     if (c->h_buf) cudaFreeHost(c->h_buf);
+    for (pcf_ctx::Lane& l : c->lane) {
+      if (l.stream) cudaStreamDestroy(l.stream);
+      if (l.join) cudaEventDestroy(l.join);
+    }
+    if (c->lane_fork) cudaEventDestroy(c->lane_fork);
     cudaStreamDestroy(c->stream);
     if (c == g_default_ctx) g_default_ctx = nullptr;
     delete c;

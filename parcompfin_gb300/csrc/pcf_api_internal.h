@@ -34,6 +34,15 @@ struct pcf_ctx {
   size_t binom_off[5] = {};  // offsets of prefix sums, tie offsets, ties, stirlerr, 2^(-j/256)
   // Serving slots of pcf_serve_trace, kept between calls (pcf_server.cpp).
   void* serve = nullptr;
+  // Streams beside `stream` for the groups of a batch on this context, made by
+  // the first plan of several groups (pcf_batch.cpp).
+  struct Lane {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t join = nullptr;
+  };
+  Lane lane[2];
+  cudaEvent_t lane_fork = nullptr;
+  int lanes = 0;
   // Upper bound on device bytes this context may hold (0 = unlimited).
   size_t budget_bytes = 0;
   // Test hook (pcf_ctx_set_test_barrier): the cooperative group barriers of

@@ -88,6 +88,30 @@ int basket_group(int d, const TuneTable& t) {
 
 namespace pcf {
 
+// The context's lanes, made on first use; returns how many there are (a failure
+// leaves fewer, or none: the groups then run one after the other).
+static int ctx_lanes(pcf_ctx* c) {
+  if (!c->lane_fork &&
+      cudaEventCreateWithFlags(&c->lane_fork, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    c->lane_fork = nullptr;
+    return 0;
+  }
+  while (c->lanes < 2) {
+    pcf_ctx::Lane& l = c->lane[c->lanes];
+    if (!l.stream && cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking) != cudaSuccess)
+      l.stream = nullptr;
+    if (!l.join && cudaEventCreateWithFlags(&l.join, cudaEventDisableTiming) != cudaSuccess)
+      l.join = nullptr;
+    if (!l.stream || !l.join) {
+      cudaGetLastError();
+      break;
+    }
+    ++c->lanes;
+  }
+  return c->lanes;
+}
+
 int plan_build(pcf_ctx* c, int n, const pcf_mc_request* reqs, cudaStream_t s, ExtMem* mem,
                pcf_plan** out, const long long* path0) {
   *out = nullptr;
@@ -313,32 +337,17 @@ int plan_build(pcf_ctx* c, int n, const pcf_mc_request* reqs, cudaStream_t s, Ex
       p->ev_fork = p->ev_join = nullptr;
     }
   }
-  if (!mem && p->groups.size() > 1) {
+  if (s == c->stream && p->groups.size() > 1) {
     // Three streams, the group that draws most normals first. A kernel's last
     // blocks, and registers and shared memory that its own blocks cannot use,
     // then go to the next groups: baskets of 4, 16 and 64 assets x 2^22 paths
     // one after the other 534 us, on two or three streams 515, on eight 511,
     // largest first 462; mixed stream of 1000 contracts 3.58 ms, two streams
     // 3.46, three 3.44, eight 3.59 (small groups then delay the large ones).
-    // A one-shot batch, whose plan lasts one launch, creates no streams.
+    // A served batch stays on its slot's stream: the slots overlap already.
     std::stable_sort(p->groups.begin(), p->groups.end(),
                      [](const Group& a, const Group& b) { return a.draws > b.draws; });
-    // A failure here only leaves fewer lanes (or none: sequential launches).
-    if (!p->ev_fork && cudaEventCreateWithFlags(&p->ev_fork, cudaEventDisableTiming) != cudaSuccess) {
-      cudaGetLastError();
-      p->ev_fork = nullptr;
-    }
-    const size_t lanes = std::min<size_t>(2, p->groups.size() - 1);
-    while (p->ev_fork && p->lanes.size() < lanes) {
-      pcf_plan::Lane l;
-      if (cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking) != cudaSuccess ||
-          cudaEventCreateWithFlags(&l.join, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        if (l.stream) cudaStreamDestroy(l.stream);
-        break;
-      }
-      p->lanes.push_back(l);
-    }
+    p->lanes = std::min(ctx_lanes(c), (int)p->groups.size() - 1);
   }
   *out = p;
   return PCF_OK;
@@ -355,34 +364,36 @@ int plan_enqueue(pcf_plan* p) {
   }
   const bool fork = p->side && p->lsm && lsm_batch_cluster_kernels(p->lsm) > 0 &&
                     !p->groups.empty();
-  if (fork || !p->lanes.empty()) {
-    const int st = cuda_status(cudaEventRecord(p->ev_fork, p->stream), "plan fork");
-    if (st) return st;
-  }
   if (fork) {
-    int st = cuda_status(cudaStreamWaitEvent(p->side, p->ev_fork, 0), "plan fork");
+    int st = cuda_status(cudaEventRecord(p->ev_fork, p->stream), "plan fork");
+    if (!st) st = cuda_status(cudaStreamWaitEvent(p->side, p->ev_fork, 0), "plan fork");
     if (!st) st = lsm_batch_launch_clusters(c, p->lsm, p->side);
     if (!st) st = cuda_status(cudaEventRecord(p->ev_join, p->side), "plan join");
     if (st) return st;
   }
-  for (pcf_plan::Lane& l : p->lanes) {
-    const int st = cuda_status(cudaStreamWaitEvent(l.stream, p->ev_fork, 0), "plan fork");
+  if (p->lanes) {
+    int st = cuda_status(cudaEventRecord(c->lane_fork, p->stream), "plan fork");
+    for (int k = 0; k < p->lanes && !st; ++k)
+      st = cuda_status(cudaStreamWaitEvent(c->lane[k].stream, c->lane_fork, 0), "plan fork");
     if (st) return st;
   }
-  size_t turn = 0;  // group k runs on stream k mod (1 + lanes)
+  int turn = 0;  // group k runs on stream k mod (1 + lanes)
+  int failed = PCF_OK;
   for (Group& gr : p->groups) {
-    const size_t k = turn++ % (p->lanes.size() + 1);
-    int st = cuda_status(launch_mc(gr.method, gr.L, gr.grid, gr.max_d, gr.block, gr.tensor,
-                                   k ? p->lanes[k - 1].stream : p->stream),
+    const int k = turn++ % (p->lanes + 1);
+    failed = cuda_status(launch_mc(gr.method, gr.L, gr.grid, gr.max_d, gr.block, gr.tensor,
+                                   k ? c->lane[k - 1].stream : p->stream),
                          "batch kernel launch");
-    if (st) return st;
+    if (failed) break;
     c->launches += 1;
   }
-  for (pcf_plan::Lane& l : p->lanes) {
-    int st = cuda_status(cudaEventRecord(l.join, l.stream), "plan join");
-    if (!st) st = cuda_status(cudaStreamWaitEvent(p->stream, l.join, 0), "plan join");
-    if (st) return st;
+  // Joined after a failed launch too: the plan's stream covers its lanes' work.
+  for (int k = 0; k < p->lanes; ++k) {
+    int st = cuda_status(cudaEventRecord(c->lane[k].join, c->lane[k].stream), "plan join");
+    if (!st) st = cuda_status(cudaStreamWaitEvent(p->stream, c->lane[k].join, 0), "plan join");
+    if (!failed) failed = st;
   }
+  if (failed) return failed;
   if (fork) {
     const int st = cuda_status(cudaStreamWaitEvent(p->stream, p->ev_join, 0), "plan join");
     return st ? st : lsm_batch_launch_coop(c, p->lsm, p->stream);
@@ -533,11 +544,6 @@ int pcf_plan_destroy(pcf_plan* p) {
     if (p->side) {
       cudaStreamSynchronize(p->side);
       cudaStreamDestroy(p->side);
-    }
-    for (pcf_plan::Lane& l : p->lanes) {
-      cudaStreamSynchronize(l.stream);
-      cudaStreamDestroy(l.stream);
-      cudaEventDestroy(l.join);
     }
     if (p->ev_fork) cudaEventDestroy(p->ev_fork);
     if (p->ev_join) cudaEventDestroy(p->ev_join);

@@ -49,15 +49,11 @@ struct pcf_plan {
   // launches replay it. graph_mode 0 never captures.
   // Fork/join: the LSM cluster launches run on `side`, concurrently with the
   // Monte Carlo groups on `stream`, so each fills the other's tail; the groups
-  // of a plan of several (that owns its memory) take turns on `stream` and the
-  // lanes for the same reason.
+  // take turns on `stream` and `lanes` of the context's lanes for the same
+  // reason.
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  struct Lane {
-    cudaStream_t stream = nullptr;
-    cudaEvent_t join = nullptr;
-  };
-  std::vector<Lane> lanes;
+  int lanes = 0;
   int graph_mode = 1;
   long long launches_done = 0;
   bool graph_failed = false;
