@@ -12,10 +12,10 @@
 // item. The last item of a contract to finish sums that contract's partials
 // in item order and widens to FP64, so results do not depend on scheduling.
 //
-// The kernels are issue-bound (a European path is ~31 FP32/INT instructions,
-// two thirds of them Philox and Box-Muller, against 3 SFU operations), so the
-// control-variate sums are compiled in only when a launch asks for them (CV
-// template flag). Baskets of more than 16 assets run mc_basket_tc_kernel,
+// The European and Asian kernels are bound by the FMA pipe that carries the
+// Philox products (64 and 77 % busy; MUFU 56 and 65, issue 64 and 63), the
+// basket kernels by issue at few warps, so the control-variate sums are
+// compiled in only when a launch asks for them (CV template flag). Baskets of more than 16 assets run mc_basket_tc_kernel,
 // which multiplies the normals by the correlation factor on the tensor
 // cores, from the basket size the tuning table routes there (24 built in,
 // where the tensor cores start to win; below it, up to 32 assets, the
@@ -69,6 +69,16 @@ __device__ __forceinline__ void item_totals(const Moments<CV>& mo, DF* sh, DF (&
     tot[1] = t[1];
     tot[2] = tot[3] = tot[4] = DF{0.f, 0.f};
   }
+}
+
+// An item's totals and their place in the contract's sums, as a call: the
+// caller's loop keeps the registers that it would have on its own.
+template <bool CV, int NW>
+__device__ __noinline__ void finish_item_call(Moments<CV> mo, DF* sh, float2* partial,
+                                              unsigned* ticket, double* out, int items, int j) {
+  DF tot[kMoments];
+  item_totals<CV, NW>(mo, sh, tot);
+  grid_finalize_df<kMoments>(tot, partial, ticket, out, items, j);
 }
 
 __device__ __forceinline__ float payoff(const McContract& C, float S) {
@@ -497,10 +507,24 @@ mc_kernel(const __grid_constant__ McLaunch L) {
       }
       basket_item<DMAX, CV, BS>(C, j, s_fb, mo);
     }
-    DF tot[kMoments];
-    item_totals<CV, BS / 32>(mo, sh, tot);
-    grid_finalize_df<kMoments>(tot, (float2*)L.partial + (size_t)base * kMoments, L.tickets + c,
-                               L.out + (size_t)c * kMoments, C.items, j);
+    // The Asian step loop fills its 64 registers, and how the sums behind it are
+    // compiled changes it: 256 contracts with the control variate take 20.46 ms
+    // with block_sum_df inlined, 20.00 with butterflies, 19.71 as a call; one
+    // contract of 10^6 x 200 without it 193, 187 and 191 us.
+    float2* const part = (float2*)L.partial + (size_t)base * kMoments;
+    double* const sums = L.out + (size_t)c * kMoments;
+    if (METHOD == MC_ASIA && CV) {
+      finish_item_call<CV, BS / 32>(mo, sh, part, L.tickets + c, sums, C.items, j);
+    } else {
+      DF tot[kMoments];
+      if (METHOD == MC_ASIA) {
+        DF v[kMoments] = {df_of(mo.y), df_of(mo.yy), df_of(mo.g), df_of(mo.gg), df_of(mo.yg)};
+        block_sum_butterfly_df<kMoments>(v, sh, tot);
+      } else {
+        item_totals<CV, BS / 32>(mo, sh, tot);
+      }
+      grid_finalize_df<kMoments>(tot, part, L.tickets + c, sums, C.items, j);
+    }
     if (threadIdx.x == 0) s_c = -1;  // every thread read s_c before block_sum_df's barriers
     __syncthreads();
   }
@@ -525,8 +549,8 @@ mc_kernel(const __grid_constant__ McLaunch L) {
 // swizzle: 8-row x 16-byte core matrices, adjacent along K 128 bytes apart
 // (leading offset) and along M/N (K/4) x 128 bytes apart (stride offset).
 //
-// What bounds it is issue: 0.6 of the slots busy, no pipe above 0.46 (ALU;
-// tensor pipe 0.18), the rest waits of few warps on one another. Baskets of 4,
+// What bounds it is the latency of few warps (15 an SM): 0.51 of the issue slots
+// are busy, ALU 0.41, MUFU and FMA 0.36, tensor pipe 0.23. Baskets of 4,
 // 16 and 64 assets, 2^22 paths each, of which this kernel was 548 us: 709 us
 // with two 8-asset buffers and four CTAs an SM; 652 with one (five CTAs fit);
 // 625 with TF32 rounding on the integer pipe instead of cvt.rna.tf32; 584 with

@@ -45,9 +45,9 @@ struct pcf_ctx {
   int lanes = 0;
   // Upper bound on device bytes this context may hold (0 = unlimited).
   size_t budget_bytes = 0;
-  // Test hook (pcf_ctx_set_test_barrier): the cooperative group barriers of
-  // pcf_mc_amer and pcf_binom_vanilla expect this many arrivals beyond their
-  // grid, so they cannot complete, and give up after test_poll_limit polls.
+  // Test hook (pcf_ctx_set_test_barrier): where this is not 0, pcf_mc_amer's
+  // exchange between blocks and pcf_binom_vanilla's grid barrier wait for more
+  // than their grid gives and give up after test_poll_limit polls.
   unsigned test_barrier_extra = 0;
   unsigned test_poll_limit = 0;
   long long launches = 0;

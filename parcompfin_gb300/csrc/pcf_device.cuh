@@ -249,6 +249,29 @@ __device__ __forceinline__ DF warp_sum_df(DF v) {
   return v;
 }
 
+// Sums K double-floats over the block by full butterflies; every lane of warp 0
+// gets the totals (the bits of block_sum_df). `sh` must hold 32*K DFs. More
+// additions than block_sum_df, fewer values alive.
+template <int K>
+__device__ __forceinline__ void block_sum_butterfly_df(DF (&v)[K], DF* sh, DF (&out)[K]) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = warp_sum_df(v[k]);
+  if (lane == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) sh[wid * K + k] = v[k];
+  }
+  __syncthreads();
+  if (wid == 0) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      DF x = lane < nw ? sh[lane * K + k] : DF{0.f, 0.f};
+      out[k] = warp_sum_df(x);
+    }
+  }
+  __syncthreads();
+}
+
 // Sums K <= 8 double-floats over a block of NW warps (a power of two); every
 // lane of warp 0 gets the totals. `sh` must hold NW*K DFs. Deterministic: a
 // butterfly over the lanes, then one over the warps. Both are reduce-scatters:
