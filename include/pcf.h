@@ -166,10 +166,11 @@ PCF_API int pcf_mc_amer_audit(pcf_ctx* ctx, double S0, double E, double r, doubl
                               double* sums, unsigned short* tau, float* u);
 
 /* Test hook for the failure paths (no counterpart in the reference): while
- * extra_arrivals > 0, the cooperative group barriers of pcf_mc_amer (plain
- * cooperative grid only: the cluster forms are not used while it is set) and
- * pcf_binom_vanilla wait for extra_arrivals blocks more than the grid holds,
- * so they cannot complete, and give up after poll_limit polls; the call then
+ * extra_arrivals > 0, the exchange between the blocks of pcf_mc_amer (plain
+ * cooperative grid only: the cluster forms are not used while it is set) waits
+ * for a total that no block publishes and the grid barrier of
+ * pcf_binom_vanilla for extra_arrivals blocks more than the grid holds, so
+ * they cannot complete, and give up after poll_limit polls; the call then
  * returns PCF_ETIMEOUT. Waits on bulk copies keep their full limit, so no
  * block leaves with a copy in flight. extra_arrivals = 0 restores normal
  * operation; the counters are reset by every call. */
@@ -200,7 +201,8 @@ PCF_API int pcf_binom_embar_batch(pcf_ctx* ctx, int n, const pcf_binom_contract*
  * Replaces double binom(S0,E,r,sigma,T,N,payoff_fun) of
  * src/binom_vanilla_eur.cpp:5-39 (american = 0) and
  * src/binom_vanilla_amer.cpp:5-40 (american = 1): bit for bit the reference's
- * FP64 result. One cooperative launch; 1 <= N <= 2,000,000. */
+ * FP64 result, in one launch (two from about 87,000 levels on);
+ * 1 <= N <= 2,000,000. */
 PCF_API int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, double sigma,
                               double T, int N, int payoff_fun, int american, double* price);
 
