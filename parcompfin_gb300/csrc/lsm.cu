@@ -181,6 +181,21 @@ __host__ __device__ __forceinline__ size_t exchange_bytes(int PB, int nblocks) {
   return exchange_fits(PB, nblocks) ? 0 : ((size_t)nblocks + 1) * kRegSums * sizeof(DF);
 }
 
+// df_add for chains of dependent additions, the same bits in fewer dependent
+// steps (6 instead of 8): the exact error of the sum from the larger operand
+// (Dekker's FastTwoSum, which is exact where |big| >= |small|), whose selection
+// runs beside the sum. A date on the cooperative grid adds 25 block totals one
+// after the other (one put of 10^5 paths x 200 dates 580 -> 567 us).
+__device__ __forceinline__ DF df_add_chain(DF a, DF b) {
+  const float s = a.hi + b.hi;
+  const bool swap = fabsf(a.hi) < fabsf(b.hi);
+  const float big = swap ? b.hi : a.hi, small = swap ? a.hi : b.hi;
+  float e = small - (s - big);
+  e += a.lo + b.lo;
+  const float hi = s + e;
+  return DF{hi, e - (hi - s)};
+}
+
 // Static shared memory of one block of NW warps: the exchange of regression
 // sums.
 template <int NW>
@@ -348,8 +363,8 @@ __device__ __forceinline__ DF block_total(const LsmShared<NW>& X) {
   DF v = DF{X.wpart[lane >> 3][q], 0.f};
 #pragma unroll
   for (int w = (lane >> 3) + 4; w < NW; w += 4) v = df_add_f(v, X.wpart[w][q]);
-  v = df_add(v, shfl_xor_df(v, 8));
-  return df_add(v, shfl_xor_df(v, 16));
+  v = df_add_chain(v, shfl_xor_df(v, 8));
+  return df_add_chain(v, shfl_xor_df(v, 16));
 }
 
 // Sum over r = 0 .. n-1 of t[r][q], q = lane & 7, in every lane of a warp: lane
@@ -371,12 +386,12 @@ __device__ __forceinline__ DF sum_totals(const DF* t, int n) {
     for (int i = 0; i < 4; ++i) y[i] = row(r + 4 * i);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      g = df_add(g, x[i]);
+      g = df_add_chain(g, x[i]);
       x[i] = y[i];
     }
   }
-  g = df_add(g, shfl_xor_df(g, 8));
-  return df_add(g, shfl_xor_df(g, 16));
+  g = df_add_chain(g, shfl_xor_df(g, 8));
+  return df_add_chain(g, shfl_xor_df(g, 16));
 }
 
 // Exchange of the CTAs' totals within a cluster, by warp 0: every CTA stores
@@ -401,9 +416,9 @@ __device__ __forceinline__ DF cluster_total(const LsmParams& P, LsmShared<NW>& X
   }
   xph ^= 1u << slot;
   DF g{0.f, 0.f};
-  for (int r = lane >> 3; r < CL; r += 4) g = df_add(g, X.xin[slot][r][q]);
-  g = df_add(g, shfl_xor_df(g, 8));
-  return df_add(g, shfl_xor_df(g, 16));
+  for (int r = lane >> 3; r < CL; r += 4) g = df_add_chain(g, X.xin[slot][r][q]);
+  g = df_add_chain(g, shfl_xor_df(g, 8));
+  return df_add_chain(g, shfl_xor_df(g, 16));
 }
 
 // Date d's normal equations from the contract's sums g (lane q's sum in every
@@ -444,10 +459,10 @@ __device__ __forceinline__ void solve_date(const LsmParams& P, LsmShared<NW>& X,
   const DF o2 = shfl_df(g, (0x102213 >> sh) & 7), o3 = shfl_df(g, (0x132243 >> sh) & 7);
   const int y0 = q < 3 ? 5 : 0;
   const DF ya = shfl_df(g, y0), yb = shfl_df(g, y0 + 1), yc = shfl_df(g, y0 + 2);
-  const DF cof = df_add(df_mul(o0, o1), df_neg(df_mul(o2, o3)));
+  const DF cof = df_add_chain(df_mul(o0, o1), df_neg(df_mul(o2, o3)));
   const DF k0 = shfl_df(cof, (0x0210 >> sh) & 7), k1 = shfl_df(cof, (0x1431 >> sh) & 7);
   const DF k2 = shfl_df(cof, (0x2542 >> sh) & 7);
-  const DF dot = df_add(df_add(df_mul(k0, ya), df_mul(k1, yb)), df_mul(k2, yc));
+  const DF dot = df_add_chain(df_add_chain(df_mul(k0, ya), df_mul(k1, yb)), df_mul(k2, yc));
   const float det = __shfl_sync(0xffffffffu, dot.hi, 3);
   int mode = 2;
   if (n == 0.f) mode = 0;
@@ -891,7 +906,7 @@ __device__ void lsm_body(const LsmParams& P, int b, int rank) {
       for (int q = 0; q < kMoments; ++q) t[q] = DF{0.f, 0.f};
       for (int r = 0; r < P.nblocks; ++r) {
         const DF* rf = cg::this_cluster().map_shared_rank(&X.fin[0], r);
-        for (int q = 0; q < kMoments; ++q) t[q] = df_add(t[q], rf[q]);
+        for (int q = 0; q < kMoments; ++q) t[q] = df_add_chain(t[q], rf[q]);
       }
       for (int q = 0; q < kMoments; ++q) P.out[q] = df_value(t[q]);
     }
@@ -1312,8 +1327,8 @@ size_t stream_state_bytes(long long Hp) { return a256(8 * (size_t)Hp) + a256(4 *
 // cooperative grid is G blocks of `smem` bytes: as many clusters of 8 (else 4)
 // CTAs as the device co-schedules, which cluster placement can make fewer
 // than the SMs. hcl = 0 when the plain cooperative kernel should run. Measured
-// on one put, 50 dates: 2^19 paths 0.40 -> 0.33 ms, 2^20 0.46 -> 0.39, 2^21
-// 0.62 -> 0.53.
+// on one put, 50 dates, plain grid against this: 2^19 paths 191 against 179 us,
+// 2^20 252 against 223, 2^21 362 against 338.
 void hybrid_shape(const LsmLimits& Lm, long long H, int M, int G, size_t smem, int& hcl, int& Gh,
                   int& PBh) {
   hcl = Gh = PBh = 0;
@@ -1339,8 +1354,9 @@ void hybrid_shape(const LsmLimits& Lm, long long H, int M, int G, size_t smem, i
     const int g = std::min((G + cl - 1) / cl, ncl) * cl;
     if (g < 2 * cl || g * 5 < G * 4) continue;  // keep at least 80 % of the grid
     const int pb = (int)(((H + g - 1) / g + 3) & ~3LL);
-    // Below ~1024 pairs per CTA the in-cluster exchange costs more than the
-    // global barrier it spares (measured: 2^17 paths 0.32 -> 0.38 ms).
+    // Below 1024 pairs per CTA the plain grid stays, although the clusters are
+    // no longer slower there (2^17 paths 167 us plain, 155 so): they add the
+    // totals in another order, which moves a coefficient's last bit.
     if (pb < 1024 || !lsm_fits(Lm, pb, M, 2, Lm.stat_coop, 1)) continue;
     hcl = cl;
     Gh = g;
