@@ -30,9 +30,11 @@ struct TuneTable {
   int basket_block[4] = {256, 256, 256, 256};
   int basket_ppt[4] = {16, 8, 8, 4};  // paths per thread per item
   int tc_tiles[2] = {8, 8};           // 128-path tiles per item, tensor-core kernel (d <= 32, <= 64)
-  // Baskets of at least this many assets take the tensor cores: measured at
-  // 2^21 paths, the CUDA cores win at 17 and 20 assets, the tensor cores from
-  // 24 on.
+  // Baskets of at least this many assets take the tensor cores: of four
+  // contracts of 2^21 paths with the control variate, one takes 74 us on the CUDA
+  // cores and 84 on the tensor cores at 17 and 20 assets, 87 and 83 at 22 and
+  // 24, 102 and 102 at 28, 117 and 101 at 32. (22 and 23 stay on the CUDA cores:
+  // the two kernels round differently.)
   int tc_min_d = 24;
   // Longstaff-Schwartz cluster launch: 0 takes the smallest cluster whose
   // CTAs cover the contract two to an SM; +1 doubles the cluster (half the
