@@ -93,6 +93,21 @@ def test_american_batch_long_and_mixed_dates_against_twin(orc, ctx):
         assert list(alone.sums) == list(r.sums), M
 
 
+@pytest.mark.parametrize("M", [1023, 1024, 1025])
+def test_american_batch_more_dates_than_slots(orc, ctx, M):
+    """512 pairs leave room for the control variate's per-date terms of 1024
+    dates; beyond that they are computed per path. Against the FP64 twin: one
+    exercise that rounding decides otherwise moves a path by at most the strike's
+    tenth, 10 of a sum of about 1024 x 8, so three of them stay below 4e-3."""
+    import parcompfin_gb300 as pcf
+    q = pcf.request("amer", 100, 100, .05, .25, 1.0, 1024, "put", M=M, seed=17, use_cv=True)
+    r = pcf.price_batch([q], ctx=ctx)[0]
+    s = (C.c_double * 6)()
+    orc.twin_mc_amer(100, 100, .05, .25, 1.0, 1024, M, -1, 0, 17, 0, s)
+    for k in (0, 2):
+        assert abs(r.sums[k] - s[k]) <= 4e-3 * abs(s[k]), (k, r.sums[k], s[k])
+
+
 def test_american_batch_against_lattice(orc, ctx):
     import parcompfin_gb300 as pcf
     reqs = [pcf.request("amer", 100, E, .05, .3, 1.0, 1 << 17, "put", M=50, use_cv=True, seed=9,
