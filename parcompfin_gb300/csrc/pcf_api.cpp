@@ -104,7 +104,8 @@ int run_mc(pcf_ctx* c, McMethod m, const McContract& k, const std::vector<float>
   if (!c->d_ticket) {
     st = cuda_status(cudaMalloc((void**)&c->d_ticket, 256), "cudaMalloc(ticket)");
     if (st) return st;
-    st = cuda_status(cudaMemset(c->d_ticket, 0, 256), "memset ticket");
+    // On the launch's own stream: nothing orders the default stream before it.
+    st = cuda_status(cudaMemsetAsync(c->d_ticket, 0, 256, c->stream), "memset ticket");
     if (st) {
       cudaFree(c->d_ticket);
       c->d_ticket = nullptr;

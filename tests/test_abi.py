@@ -124,3 +124,22 @@ def test_binom_batch_packing_matches_field_by_field():
             api._pack_binom(bad)
     with pytest.raises(TypeError):
         api._pack_binom([(1, "2", 3, 4, 5, 6, "put")])
+
+
+def _csrc_calls(pattern):
+    """(file, line, text) of the lines of csrc that match."""
+    csrc = os.path.join(ROOT, "parcompfin_gb300", "csrc")
+    hits = []
+    for f in sorted(os.listdir(csrc)):
+        for k, line in enumerate(open(os.path.join(csrc, f)), 1):
+            if re.search(pattern, line.split("//")[0]):
+                hits.append((f, k, line.strip()))
+    return hits
+
+
+def test_no_memset_on_the_default_stream():
+    """Contexts run on non-blocking streams, which the default stream does not
+    wait for and which do not wait for it: a cudaMemset is ordered with no
+    launch. Every clear is a cudaMemsetAsync on the stream of its launch."""
+    assert _csrc_calls(r"\bcudaMemset\s*\(") == []
+    assert _csrc_calls(r"\bcudaMemsetAsync\s*\(")

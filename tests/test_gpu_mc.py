@@ -286,3 +286,30 @@ def test_basket_book_full_size_matches_fp64_twin(orc, ctx):
                            c["N"], 1, 11, i, s)
         for k in range(5):
             assert rel(r.sums[k], s[k]) < DET_REL, (d, k, r.sums[k], s[k])
+
+
+def test_first_single_call_beside_a_busy_default_stream(ctx):
+    """A context's first single-contract call, and the first after a release,
+    clear the ticket word on the context's own stream: with work queued on the
+    default stream, and device memory that holds other launches' leavings, the
+    sums are those of any later call."""
+    torch = pytest.importorskip("torch")
+    from parcompfin_gb300 import Context, mc_asia_result, mc_basket_result, mc_eur_result
+    calls = [lambda c: mc_eur_result(100, 95, .05, .2, 1, 100_003, 1, seed=3, use_cv=True, ctx=c),
+             lambda c: mc_asia_result(100, 95, .05, .2, 1, 20_000, 12, 1, seed=3, ctx=c),
+             lambda c: mc_basket_result([100.0] * 4, [.2] * 4, [float(i % 5 == 0) for i in range(16)],
+                                        .05, 1.0, 100.0, 50_000, 1, seed=9, ctx=c)]
+    for call in calls:
+        want = list(call(ctx).sums)
+        with Context(0) as c:
+            for _ in range(2):
+                dirty = [torch.full((n,), -1, dtype=torch.int32, device="cuda")
+                         for n in (64, 1 << 18, 1 << 20)]
+                torch.cuda.synchronize()
+                del dirty
+                torch.cuda.empty_cache()
+                torch.cuda._sleep(100_000_000)  # about 50 ms on the default stream
+                assert list(call(c).sums) == want
+                torch.cuda.synchronize()
+                assert list(call(c).sums) == want
+                c.release()
