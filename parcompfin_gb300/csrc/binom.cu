@@ -837,7 +837,13 @@ int ensure_tables(pcf_ctx* c, int nmax) {
   for (int j = 0; j < 256; ++j)  // 2^(-j/256) in units of 2^-63
     ((unsigned long long*)&h[o_exp2])[j] =
         (unsigned long long)roundl(ldexpl(exp2l(-(long double)j / 256), 63));
-  st = cuda_status(cudaMemcpy(d, h.data(), total, cudaMemcpyHostToDevice), "H2D binomial tables");
+  // On the context's stream and waited for: a copy from pageable memory on the
+  // default stream may still be on its way when the call returns, and nothing
+  // orders it before this stream's launches.
+  st = cuda_status(cudaMemcpyAsync(d, h.data(), total, cudaMemcpyHostToDevice, c->stream),
+                   "H2D binomial tables");
+  const int landed = cuda_status(cudaStreamSynchronize(c->stream), "H2D binomial tables");
+  if (!st) st = landed;
   if (st) {
     cudaFree(d);
     return st;

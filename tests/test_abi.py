@@ -143,3 +143,11 @@ def test_no_memset_on_the_default_stream():
     launch. Every clear is a cudaMemsetAsync on the stream of its launch."""
     assert _csrc_calls(r"\bcudaMemset\s*\(") == []
     assert _csrc_calls(r"\bcudaMemsetAsync\s*\(")
+
+
+def test_no_copy_on_the_default_stream():
+    """A plain cudaMemcpy from pageable memory may return before its transfer
+    to the device is done, and no context's stream waits for it: copies are
+    queued on the stream of the launches that read them."""
+    assert _csrc_calls(r"\bcudaMemcpy\s*\(") == []
+    assert _csrc_calls(r"\bcudaMemcpyAsync\s*\(")

@@ -232,3 +232,20 @@ def test_accurate_mode_matches_exact_decimals(orc, ctx, N):
         ref = _exact_binom(orc, 100.0, 105.0, r, sig, T, N, pf)
         v = binom_embar(100.0, 105.0, r, sig, T, N, pf, mode="accurate", ctx=ctx)
         assert abs(v - ref) <= EXACT_TOL * abs(ref), (N, r, v, ref)
+
+
+def test_first_tables_beside_a_busy_default_stream(ctx):
+    """A context's first sum uploads its tables on the context's own stream and
+    waits for them, whatever the default stream has queued; so do larger
+    tables and the tables after a release."""
+    torch = pytest.importorskip("torch")
+    from parcompfin_gb300 import Context, binom_embar
+    args = (100.0, 105.0, .03, .3, 1.5)
+    want = {N: binom_embar(*args, N, -1, ctx=ctx) for N in (1000, 50_000)}
+    with Context(0) as c:
+        for _ in range(2):
+            for N in (1000, 50_000):
+                torch.cuda._sleep(100_000_000)  # about 50 ms on the default stream
+                assert binom_embar(*args, N, -1, ctx=c) == want[N]
+                torch.cuda.synchronize()
+            c.release()
