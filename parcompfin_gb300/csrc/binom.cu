@@ -95,7 +95,7 @@ struct BinomTables {
 struct BinomContract {
   double S0, E, u, d, lp, lq, logu, logd;
   double p, q;   // accurate mode
-  double lpq, stirl_n, twopi_n;  // accurate mode: log(p / q), stirlerr(N), 2 pi / N
+  double stirl_n, twopi_n;  // accurate mode: stirlerr(N), 2 pi / N
   int N, pf, i_lo, i_hi;  // pair indices i_lo..i_hi (inclusive)
   int has_mid, items, terms;
   int wide;      // a power of u or d may leave the FP64 range: binom_wide_kernel prices it
@@ -109,6 +109,8 @@ struct BinomPrep {
   // of its mirror S0 u^(N-i) d^i is y2 - i dy: signed 128-bit numbers (high,
   // low word) with 96 bits after the point.
   unsigned long long y1[2], y2[2], dy[2];
+  // Accurate mode: -|log(p / (1 - p))|, high and low part.
+  double ratio[2];
   // The accumulator of comb() after + log N .. + log(n + 1) at the stretch
   // starts n = seg_n[0] (the largest index of the window) > seg_n[1] > ...
   int segs, cut;           // cut: more stretches than kSegs, the last one goes on
@@ -653,14 +655,16 @@ __global__ void __launch_bounds__(kPrepBlock) binom_prep_kernel(BinomLaunch L) {
   for (int k = lane; k < C.items; k += 32) L.item_contract[L.item_start[c] + k] = c;
   if (lane == 0) L.tickets[c] = 0u;
   if (C.wide) return;
-  const __int128 g = lane < 3 ? log2_q96(lane == 0 ? C.u : lane == 1 ? C.d : C.S0) : 0;
+  // (lanes 3 and 4 for the accurate mode)
+  const double arg = lane == 0 ? C.u : lane == 1 ? C.d : lane == 2 ? C.S0 : lane == 3 ? C.p : C.q;
+  const __int128 g = lane < (L.mode ? 5 : 3) ? log2_q96(arg) : 0;
   unsigned long long gh = (unsigned long long)(g >> 64), gl = (unsigned long long)g;
   auto from = [&](int src) {
     const unsigned long long h = __shfl_sync(0xffffffffu, gh, src);
     const unsigned long long l = __shfl_sync(0xffffffffu, gl, src);
     return (__int128)(((unsigned __int128)h << 64) | l);
   };
-  const __int128 lu = from(0), ld = from(1), ls = from(2);
+  const __int128 lu = from(0), ld = from(1), ls = from(2), lp = from(3), lq = from(4);
   if (lane == 0) {
     auto put = [](unsigned long long (&w)[2], __int128 v) {
       w[0] = (unsigned long long)(v >> 64);
@@ -669,6 +673,18 @@ __global__ void __launch_bounds__(kPrepBlock) binom_prep_kernel(BinomLaunch L) {
     put(R->y1, ls + C.N * ld);
     put(R->y2, ls + C.N * lu);
     put(R->dy, lu - ld);
+    if (L.mode) {
+      // |log2(p/q)| ln 2, still in units of 2^-96, as a sum of two doubles. q is
+      // 1 - p rounded: log(1 - p) = log q + (1 - q - p)/q.
+      const unsigned __int128 a = lp > lq ? lp - lq : lq - lp;
+      const unsigned long long ln2 = 0xB17217F7D1CF79ACULL;  // ln 2 2^64
+      const unsigned __int128 v = (a >> 64) * ln2 + __umul64hi((unsigned long long)a, ln2);
+      const double hi = (double)(long long)(v >> 46);  // below 2^60
+      const long long lo = (long long)((__int128)v - ((__int128)(long long)hi << 46));
+      const double dq = __ddiv_rn(__dsub_rn(__dsub_rn(1.0, C.q), C.p), C.q);
+      R->ratio[0] = -hi * 0x1p-50;
+      R->ratio[1] = -((double)lo * 0x1p-96) + (lp > lq ? dq : -dq);
+    }
   }
 }
 
@@ -725,9 +741,17 @@ __global__ void __launch_bounds__(kBinomBlock) binom_kernel(BinomLaunch L) {
       b1 = __dadd_rn(__dadd_rn(cv, __dmul_rn(di, C.lp)), __dmul_rn(dj, C.lq));
       b2 = __dadd_rn(__dadd_rn(cv, __dmul_rn(dj, C.lp)), __dmul_rn(di, C.lq));
     } else {
-      // The mirrored weight C(N,i) p^(N-i) q^i is the first times (p/q)^(N-2i).
-      b1 = log_dbinom_shared(i, C, C.stirl_n, L.stirl);
-      b2 = __fma_rn((double)(N - 2 * i), C.lpq, b1);
+      // The larger weight of the pair by its own logarithm, the smaller one from
+      // it: their ratio is ((1-p)/p)^(N-2i) where p > 1/2. Both terms of the sum
+      // are negative, so it is as good as the smaller weight's own logarithm; the
+      // larger one from the smaller would carry the smaller's absolute error
+      // (1e-12 of the price at N = 50,001 and p = 0.64).
+      const bool up = __double_as_longlong(C.p) > __double_as_longlong(C.q);
+      const double b = log_dbinom_shared(up ? N - i : i, C, C.stirl_n, L.stirl);
+      const double n2 = small_to_double(N - 2 * i);
+      const double m = __fma_rn(n2, R.ratio[1], __fma_rn(n2, R.ratio[0], b));
+      b1 = up ? m : b;
+      b2 = up ? b : m;
     }
     const unsigned __int128 iy = u128(R.dy) * (unsigned)i;
     const double s1 = exp2_q96(u128(R.y1) + iy, T), s2 = exp2_q96(u128(R.y2) - iy, T);
@@ -883,7 +907,6 @@ int setup_contract(const pcf_binom_contract& k, int idx, BinomContract& C) {
   C.lq = log(q);
   C.logu = log(u);
   C.logd = log(d);
-  C.lpq = log1p((p - q) / q);
   C.twopi_n = 2 * 3.14159265358979323846 / N;
   if (N <= 15) {
     double small[16];

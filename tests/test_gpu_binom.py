@@ -249,3 +249,23 @@ def test_first_tables_beside_a_busy_default_stream(ctx):
                 assert binom_embar(*args, N, -1, ctx=c) == want[N]
                 torch.cuda.synchronize()
             c.release()
+
+
+@pytest.mark.parametrize("r,sig,T,N", [(.06, .02, 2.0, 2001), (.1, .02, 5.0, 20_001),
+                                       (.1, .005, 10.0, 50_001), (.05, .01, 1.0, 30_000)])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_accurate_mode_away_from_even_odds(orc, ctx, r, sig, T, N, sign):
+    """Drifts of 3 to 20 volatilities, p above and below 1/2: of a pair's two weights
+    either may be the one that matters, also for a payoff that only the smaller
+    one has (strikes at the forward and three deviations to both sides).
+    Bound: N p and N q are rounded, which moves a weight's logarithm by
+    |k - N p| 2^-53 each; within four deviations, |k - N p| <= 2 sqrt(N). Eight
+    more units for the logarithm's other terms, the powers and the sum."""
+    from parcompfin_gb300 import binom_embar_batch
+    r *= sign
+    forward = 100.0 * math.exp(r * T)
+    cs = [(100.0, forward * math.exp(k * sig * math.sqrt(T)), r, sig, T, N, pf)
+          for k in (-3, 0, 3) for pf in (1, -1)]
+    for c, v in zip(cs, binom_embar_batch(cs, mode="accurate", ctx=ctx)):
+        ref = _exact_binom(orc, *c)
+        assert abs(v - ref) <= (8 + 2 * math.sqrt(N)) * 2**-52 * ref, (c, v, ref, rel(v, ref))
