@@ -448,6 +448,24 @@ __global__ void __launch_bounds__(kLatBlock) lattice_kernel(LatticeParams P, int
   }
 }
 
+// Whether a node may be infinite or not a number where the fast strips would
+// lose it: they take a payoff's sign, and an American node's larger value, from
+// the bits, and their division turns an infinite node into a NaN of either sign.
+//   put       S0 u^i = inf where d^(n-i) = 0 is a NaN share price; other
+//             infinite share prices have payoff 0;
+//   American  every value, at most the largest payoff grown by R^-N, has to be
+//             finite. (European strips compare nothing: what is not finite
+//             reaches the root, and that is computed again.)
+bool lat_leaves_range(double S0, double E, double R, int N, int pf, bool american,
+                      const double* up, const double* dn) {
+  if (pf < 0 && !std::isfinite(S0 * up[N]))
+    for (int i = N; i >= 0 && !std::isfinite(S0 * up[i]); --i)
+      if (dn[N - i] == 0.0) return true;
+  if (!american) return false;
+  const double top = (pf > 0 ? S0 * std::max(1.0, up[N]) * std::max(1.0, dn[N]) : 0.0) + E;
+  return !(top * std::max(1.0, pow(1.0 / R, (double)N)) < 0x1p1023);
+}
+
 typedef void (*StripKernel)(LatticeParams);
 StripKernel strip_kernel(bool amer, bool exact, bool help) {
   if (!amer) return exact ? lattice_strip_kernel<false, true, false> : lattice_strip_kernel<false, false, false>;
@@ -473,7 +491,8 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
     double u, d, p, q, R;
     lattice(r, sigma, T, N, u, d, p, q, R);
     // The ordinary range of the three-operation division and of comparing
-    // node values as integers (all of them non-negative and finite).
+    // node values as integers (all of them non-negative and finite: see
+    // lat_leaves_range).
     bool exact = !(R >= 0.5 && R <= 2.0 && p > 0 && p < 1 && q > 0);
 
     // Strips from level `top`: the level N, or the largest that fits.
@@ -522,6 +541,7 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
       h[i] = pow(u, (double)i);
       h[nodes + i] = pow(d, (double)i);
     }
+    exact = exact || lat_leaves_range(S0, E, R, N, payoff_fun, american != 0, h, h + nodes);
     st = cuda_status(cudaMemcpyAsync(dv + o_up, h, 16 * nodes, cudaMemcpyHostToDevice, c->stream),
                      "H2D lattice tables");
     if (st) return st;

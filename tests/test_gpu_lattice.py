@@ -83,3 +83,31 @@ def test_lattice_division_range_bit_exact(orc, ctx, args, american):
     fn = pcf.binom_vanilla_amer if american else pcf.binom_vanilla_eur
     ref = orc.ref_binom_vanilla_amer if american else orc.ref_binom_vanilla_eur
     assert fn(*args, ctx=ctx) == ref(*args[:6], float(args[6]))
+
+
+def _same(a, b):
+    return a == b or (a != a and b != b)
+
+
+# Lattices whose powers or values leave the FP64 range. (S0, E, r, sigma, T, N):
+OUT_OF_RANGE = {
+    "inf-times-0": (100, 100, .03, 20.0, 4.0, 1000),     # S0 u^i = inf and d^(N-i) = 0: NaN nodes
+    "inf": (100, 100, .03, 18.0, 1.0, 1500),             # S0 u^N = inf alone
+    "growing": (100, 1e200, -260.0, 25.3, 1.0, 400),     # R = 0.52: E R^-N overflows
+    "zero-d": (100, 100, .03, 30.0, 1.0, 20),            # d rounds to 0
+    "zero-d-inf": (100, 100, .03, 60.0, 1.0, 40),
+}
+
+
+@pytest.mark.parametrize("american", [False, True])
+@pytest.mark.parametrize("pf", [1, -1])
+@pytest.mark.parametrize("name", OUT_OF_RANGE)
+def test_lattice_out_of_range_nodes(orc, ctx, name, pf, american):
+    """Infinite and not-a-number nodes go where the reference's operations take
+    them: the same price, infinite or not a number included."""
+    import parcompfin_gb300 as pcf
+    fn = pcf.binom_vanilla_amer if american else pcf.binom_vanilla_eur
+    ref = orc.ref_binom_vanilla_amer if american else orc.ref_binom_vanilla_eur
+    args = OUT_OF_RANGE[name]
+    got, want = fn(*args, pf, ctx=ctx), ref(*args, float(pf))
+    assert _same(got, want), (name, pf, american, got, want)
