@@ -168,13 +168,23 @@ PCF_API int pcf_mc_amer_audit(pcf_ctx* ctx, double S0, double E, double r, doubl
 /* Test hook for the failure paths (no counterpart in the reference): while
  * extra_arrivals > 0, the exchange between the blocks of pcf_mc_amer (plain
  * cooperative grid only: the cluster forms are not used while it is set) waits
- * for a total that no block publishes and the grid barrier of
- * pcf_binom_vanilla for extra_arrivals blocks more than the grid holds, so
- * they cannot complete, and give up after poll_limit polls; the call then
- * returns PCF_ETIMEOUT. Waits on bulk copies keep their full limit, so no
- * block leaves with a copy in flight. extra_arrivals = 0 restores normal
- * operation; the counters are reset by every call. */
+ * for a total that no block publishes; in pcf_binom_vanilla the grid barrier
+ * of the levels above the strips waits for extra_arrivals blocks more than the
+ * grid holds and the strips are starved as by pcf_ctx_set_test_lattice(2)
+ * (one strip, N < 24, waits for nothing). So they cannot complete, and give up
+ * after poll_limit polls; the call then returns PCF_ETIMEOUT. Waits on bulk
+ * copies keep their full limit, so no block leaves with a copy in flight.
+ * extra_arrivals = 0 restores normal operation; the counters are reset by
+ * every call. */
 PCF_API int pcf_ctx_set_test_barrier(pcf_ctx* ctx, unsigned extra_arrivals, unsigned poll_limit);
+
+/* Test hook for the strips of pcf_binom_vanilla: which of their waits to
+ * starve. 2: strip 1 publishes its nodes where nobody reads, 3: the reader of
+ * its ring reports what it has taken where nobody looks, 4: that reader stops
+ * handing the nodes on to its block. That wait gives up after poll_limit polls
+ * and the call returns PCF_ETIMEOUT, its message naming the wait. 0 restores
+ * normal operation. The lattice needs two strips, for 3 some 1100 levels. */
+PCF_API int pcf_ctx_set_test_lattice(pcf_ctx* ctx, int withhold, unsigned poll_limit);
 
 /* European option by the closed binomial sum on the reference's
  * beta-parametrised lattice (u = beta + sqrt(beta^2 - 1), d = 1/u).

@@ -77,10 +77,17 @@ class Context:
         _lib.check(_lib.load().pcf_ctx_set_memory_limit(self._h, int(nbytes)))
 
     def set_test_barrier(self, extra_arrivals: int, poll_limit: int = 1) -> None:
-        """Test hook: make the cooperative group barriers of mc_amer and the
+        """Test hook: make the waits between the blocks of mc_amer and the
         lattice pricers unable to complete (extra_arrivals > 0) so that they
         give up after poll_limit polls; 0 restores normal operation."""
         _lib.check(_lib.load().pcf_ctx_set_test_barrier(self._h, int(extra_arrivals),
+                                                         int(poll_limit)))
+
+    def set_test_lattice(self, withhold: int, poll_limit: int = 1) -> None:
+        """Test hook: starve one wait of the lattice strips (2: the right
+        neighbour's nodes, 3: the ring's reader, 4: the courier's words) so
+        that it gives up after poll_limit polls; 0 restores normal operation."""
+        _lib.check(_lib.load().pcf_ctx_set_test_lattice(self._h, int(withhold),
                                                          int(poll_limit)))
 
     def autotune(self, mc: bool = True, lsm: bool = True, save: bool = False,

@@ -82,6 +82,7 @@ constexpr int kOwn = 32 - kHalo;   // strips: columns a warp owns, a multiple of
 constexpr int kRing = 1024;        // strips: words of a ring between two blocks of threads
 constexpr int kInRing = 64;        // strips: words of the shared-memory ring
 constexpr int kRingCheck = 32;     // strips: level blocks between two overrun checks
+constexpr int kKept = 64;          // strips, test hook: words the courier hands on before it stops
 constexpr unsigned long long kEmpty = ~0ULL;  // a NaN pattern no node takes
 
 struct LatticeParams {
@@ -93,8 +94,8 @@ struct LatticeParams {
   double* B;
   unsigned* barrier;
   int* err;
-  unsigned wait_limit;
-  unsigned barrier_extra;  // test hook: arrivals the barrier expects beyond the grid
+  unsigned wait_limit;     // blocked: polls at the grid barrier before giving up
+  unsigned barrier_extra;  // blocked, test hook: arrivals the barrier expects beyond the grid
   double* out;
   // strips
   int top;                     // level the strips start from
@@ -104,7 +105,20 @@ struct LatticeParams {
   int sms;
   unsigned long long* ring;    // strips x kRing words, filled with kEmpty
   unsigned* taken;             // strips: words of the ring its reader has taken
+  unsigned word_limit;         // polls before giving up: the courier's for a neighbour's word,
+  unsigned reader_limit;       // a strip's for its ring's reader,
+  unsigned hand_limit;         // and a lane's for a word from the courier (shared memory)
+  int withhold;                // test hook: what strip 1 (kLatWord) or strip 0's courier keeps back
 };
+
+// What P.err says gave up, and the host's words for it. The first one stays.
+enum LatWait : int { kLatBarrier = 1, kLatWord = 2, kLatReader = 3, kLatHandOver = 4 };
+const char* lat_wait_name(int w) {
+  return w == kLatWord     ? "wait for the right neighbour's nodes"
+         : w == kLatReader ? "wait for the ring's reader"
+         : w == kLatHandOver ? "wait for the courier's words"
+                             : "grid barrier";
+}
 
 // include/common.h:56-60: std::max(payoff_fun * (St - E), 0.0).
 __device__ __forceinline__ double lat_payoff(const LatticeParams& P, int n, int i) {
@@ -151,6 +165,9 @@ __device__ __forceinline__ unsigned long long ring_word(double v) {
 __device__ __forceinline__ bool lat_stopped(const LatticeParams& P) {
   return *((volatile int*)P.err) != 0;
 }
+__device__ __forceinline__ void lat_give_up(const LatticeParams& P, LatWait w) {
+  atomicCAS(P.err, 0, (int)w);
+}
 
 // The courier warp of strip b: takes the words k = 0 .. words-1 from the ring
 // of strip b + 1 in batches of 32, one word per lane, empties each ring slot
@@ -160,10 +177,13 @@ __device__ void strip_courier(const LatticeParams& P, int b, int words,
                               volatile unsigned long long* in) {
   const int lane = threadIdx.x & 31;
   unsigned long long* ring = P.ring + (size_t)(b + 1) * kRing;
+  // Test hook: strip 0's courier reports where nobody looks.
+  unsigned* taken = P.taken + (P.withhold == kLatReader && b == 0 ? 0 : b + 1);
   for (int k0 = 0; k0 < words; k0 += 32) {
     const int k = k0 + lane;
     bool have = k >= words, done = have;
     unsigned long long v = kEmpty;
+  #pragma unroll 1
     for (unsigned polls = 0;; ++polls) {
       if (!have) {
         v = ring_load(ring + (k & (kRing - 1)));
@@ -177,8 +197,8 @@ __device__ void strip_courier(const LatticeParams& P, int b, int words,
         done = true;
       }
       if (__all_sync(0xffffffffu, done)) break;
-      if ((polls & 63u) == 63u && (polls > P.wait_limit || lat_stopped(P))) {
-        if (lane == 0) atomicExch(P.err, 1);
+      if ((polls & 63u) == 63u && (polls > P.word_limit || lat_stopped(P))) {
+        if (lane == 0) lat_give_up(P, kLatWord);
         return;  // the compute warps see P.err in their own wait
       }
     }
@@ -186,7 +206,7 @@ __device__ void strip_courier(const LatticeParams& P, int b, int words,
     // also empty the SM's L1, which holds the d^j).
     __syncwarp();
     if (lane == 0)
-      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(P.taken + b + 1),
+      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(taken),
                    "r"((unsigned)min(k0 + 32, words))
                    : "memory");
   }
@@ -209,10 +229,6 @@ __global__ void __launch_bounds__(32 * (kStripWarps + 1), kStripsPerSm)
   int b = blockIdx.x;
   const int row = b / P.sms, r0 = row * P.sms;
   if (row & 1) b = r0 + min(P.strips - r0, P.sms) - 1 - (b - r0);
-  if (P.barrier_extra) {  // test hook: a grid barrier that cannot complete
-    group_barrier(P.barrier, gridDim.x + P.barrier_extra, P.err, P.wait_limit);
-    return;
-  }
   const int a0 = b * C, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool right = b + 1 < P.strips;  // a strip to the right feeds this one
   for (int k = threadIdx.x; k < kInRing; k += blockDim.x) in[k] = kEmpty;
@@ -223,7 +239,9 @@ __global__ void __launch_bounds__(32 * (kStripWarps + 1), kStripsPerSm)
   const int n1 = (P.top - 1) & ~(kHalo - 1);  // the first block's last level
   if (w == W) {
     const int ar = a0 + C;  // the right strip's first column: it ends at level ar
-    if (right) strip_courier(P, b, kHalo * (1 + (P.top > ar ? (n1 - ar) / kHalo + 1 : 0)), in);
+    int words = kHalo * (1 + (P.top > ar ? (n1 - ar) / kHalo + 1 : 0));
+    if (P.withhold == kLatHandOver && b == 0) words = min(words, kKept);  // test hook
+    if (right) strip_courier(P, b, words, in);
     return;
   }
   const int meet = 32 * (HELP ? W + 1 : W);  // threads of the block's barrier
@@ -311,6 +329,7 @@ __global__ void __launch_bounds__(32 * (kStripWarps + 1), kStripsPerSm)
   double v = 0.0;
   if (i <= P.top) v = P.src ? P.src[i] : payoff_of(su, down(P.top, i));
   unsigned long long* ring = P.ring + (size_t)b * kRing;  // strip 0's is written, never read
+  if (P.withhold == kLatWord && b == 1) ring -= kRing;    // test hook: as strip 0's
   const bool edge = lane < kHalo;    // the nodes the left neighbour needs
   const bool halo = lane >= kOwn;    // the right neighbour's first nodes
   const bool fed = halo && w + 1 == W && right;
@@ -335,8 +354,8 @@ __global__ void __launch_bounds__(32 * (kStripWarps + 1), kStripsPerSm)
         // the reader must have taken.
         const int need = (kb + kRingCheck + 1) * kHalo - kRing;
         for (unsigned polls = 0; (int)*((volatile unsigned*)(P.taken + b)) < need;) {
-          if (++polls > P.wait_limit || lat_stopped(P)) {
-            atomicExch(P.err, 1);
+          if (++polls > P.reader_limit || lat_stopped(P)) {
+            lat_give_up(P, kLatReader);
             fail = 1;
             break;
           }
@@ -365,8 +384,8 @@ __global__ void __launch_bounds__(32 * (kStripWarps + 1), kStripsPerSm)
       unsigned long long x;
       const int slot = (kb * kHalo + lane - kOwn) & (kInRing - 1);
       while ((x = vin[slot]) == kEmpty) {
-        if ((++polls & 1023u) == 0 && (polls > (P.wait_limit << 6) || lat_stopped(P))) {
-          atomicExch(P.err, 1);
+        if ((++polls & 1023u) == 0 && (polls > P.hand_limit || lat_stopped(P))) {
+          lat_give_up(P, kLatHandOver);
           fail = 1;
           dead = true;
           break;
@@ -564,11 +583,16 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
     P.err = (int*)(dv + o_cnt + 64);
     P.taken = (unsigned*)(dv + o_cnt + 256);
     P.ring = (unsigned long long*)(dv + o_ring);
-    P.wait_limit = 1u << 22;
-    if (c->test_barrier_extra) {  // test hook: a barrier that cannot complete
-      P.barrier_extra = c->test_barrier_extra;
-      P.wait_limit = c->test_poll_limit;
-    }
+    P.wait_limit = P.word_limit = P.reader_limit = 1u << 22;  // seconds
+    P.hand_limit = 1u << 28;
+    // Test hooks: waits that cannot complete. Only the starved one is cut short;
+    // the others end when they see that it gave up.
+    P.barrier_extra = c->test_barrier_extra;
+    P.withhold = c->test_barrier_extra ? kLatWord : c->test_lattice;
+    if (P.barrier_extra) P.wait_limit = c->test_poll_limit;
+    if (P.withhold == kLatWord) P.word_limit = c->test_poll_limit;
+    if (P.withhold == kLatReader) P.reader_limit = c->test_poll_limit;
+    if (P.withhold == kLatHandOver) P.hand_limit = c->test_poll_limit;
     P.out = (double*)(dv + o_out);
     P.top = top;
     P.warps = W;
@@ -611,7 +635,8 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
                        "D2H lattice");
       if (!st) st = cuda_status(cudaStreamSynchronize(c->stream), "lattice kernel");
       if (st) return st;
-      if (((const int*)h)[16]) return set_error(PCF_ETIMEOUT, "lattice grid barrier gave up");
+      if (const int w = ((const int*)h)[16])
+        return set_error(PCF_ETIMEOUT, "lattice %s gave up", lat_wait_name(w));
       root = h[16];
       if (exact || (root >= 0x1p-700 && std::isfinite(root))) break;
       exact = true;  // too small (or not finite) for the three-operation division

@@ -391,6 +391,21 @@ int pcf_ctx_set_test_barrier(pcf_ctx* ctx, unsigned extra_arrivals, unsigned pol
   });
 }
 
+int pcf_ctx_set_test_lattice(pcf_ctx* ctx, int withhold, unsigned poll_limit) {
+  return pcf::abi_guard([&]() -> int {
+    int st;
+    pcf_ctx* c = resolve_ctx(ctx, &st);
+    if (!c) return st;
+    if (withhold != 0 && (withhold < 2 || withhold > 4))
+      return set_error(PCF_EINVAL, "withhold must be 0, 2, 3 or 4");
+    if (withhold && poll_limit < 1)
+      return set_error(PCF_EINVAL, "poll_limit must be >= 1 with a withheld word");
+    c->test_lattice = withhold;
+    c->test_poll_limit = withhold ? poll_limit : 0;
+    return PCF_OK;
+  });
+}
+
 int pcf_mc_eur(pcf_ctx* ctx, double S0, double E, double r, double sigma, double T, long long N,
                int payoff_fun, unsigned long long seed, int use_cv, pcf_mc_result* out) {
   return pcf::abi_guard([&]() -> int {

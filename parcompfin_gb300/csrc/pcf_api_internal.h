@@ -46,10 +46,11 @@ struct pcf_ctx {
   // Upper bound on device bytes this context may hold (0 = unlimited).
   size_t budget_bytes = 0;
   // Test hook (pcf_ctx_set_test_barrier): where this is not 0, pcf_mc_amer's
-  // exchange between blocks and pcf_binom_vanilla's grid barrier wait for more
-  // than their grid gives and give up after test_poll_limit polls.
+  // exchange between blocks and pcf_binom_vanilla's waits between blocks want
+  // more than their grid gives and give up after test_poll_limit polls.
   unsigned test_barrier_extra = 0;
   unsigned test_poll_limit = 0;
+  int test_lattice = 0;  // test hook (pcf_ctx_set_test_lattice): the wait to starve
   long long launches = 0;
 };
 

@@ -111,3 +111,30 @@ def test_lattice_out_of_range_nodes(orc, ctx, name, pf, american):
     args = OUT_OF_RANGE[name]
     got, want = fn(*args, pf, ctx=ctx), ref(*args, float(pf))
     assert _same(got, want), (name, pf, american, got, want)
+
+
+WAITS = {2: "right neighbour's nodes", 3: "ring's reader", 4: "courier's words"}
+
+
+@pytest.mark.parametrize("american", [True, False])
+@pytest.mark.parametrize("N", [1200, 4000, 9000, 20000])  # 24, 48, 72 and 96 columns a strip
+@pytest.mark.parametrize("withhold", WAITS)
+def test_lattice_starved_waits_give_up_then_recover(orc, ctx, withhold, N, american):
+    """Each bounded wait between the strips is made to run out: a strip that
+    stops publishing, a reader that stops reporting, a courier that stops
+    handing on. The call returns PCF_ETIMEOUT and names the wait, with and
+    without the warp that computes exercise values; the next call on the same
+    context gives the reference's price."""
+    import parcompfin_gb300 as pcf
+    from parcompfin_gb300._lib import PCF_ETIMEOUT, PcfError
+    fn = pcf.binom_vanilla_amer if american else pcf.binom_vanilla_eur
+    ref = orc.ref_binom_vanilla_amer if american else orc.ref_binom_vanilla_eur
+    args = CASES[0]
+    ctx.set_test_lattice(withhold, 2000)
+    try:
+        with pytest.raises(PcfError, match=WAITS[withhold]) as e:
+            fn(*args, N, -1, ctx=ctx)
+        assert e.value.status == PCF_ETIMEOUT
+    finally:
+        ctx.set_test_lattice(0)
+    assert fn(*args, N, -1, ctx=ctx) == ref(*args, N, -1.0)
