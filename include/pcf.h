@@ -186,6 +186,12 @@ PCF_API int pcf_ctx_set_test_barrier(pcf_ctx* ctx, unsigned extra_arrivals, unsi
  * normal operation. The lattice needs two strips, for 3 some 1100 levels. */
 PCF_API int pcf_ctx_set_test_lattice(pcf_ctx* ctx, int withhold, unsigned poll_limit);
 
+/* Test hook: with level > 0 the strips of pcf_binom_vanilla take over at that
+ * level at the latest, so that a lattice of a few thousand levels runs the
+ * kernel of the levels above them too (ordinarily from about 87,500 on).
+ * Prices are the same bits. 0 restores normal operation. */
+PCF_API int pcf_ctx_set_test_strip_level(pcf_ctx* ctx, int level);
+
 /* European option by the closed binomial sum on the reference's
  * beta-parametrised lattice (u = beta + sqrt(beta^2 - 1), d = 1/u).
  * Replaces double binom(S0,E,r,sigma,T,N,payoff_fun), src/binom_embar.cpp:5-50

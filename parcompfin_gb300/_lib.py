@@ -140,6 +140,7 @@ SIGNATURES = {
                                C.POINTER(C.c_ushort), C.POINTER(C.c_float)]),
     "pcf_ctx_set_test_barrier": (_I, [_P, C.c_uint, C.c_uint]),
     "pcf_ctx_set_test_lattice": (_I, [_P, _I, C.c_uint]),
+    "pcf_ctx_set_test_strip_level": (_I, [_P, _I]),
     "pcf_autotune": (_I, [_P, _I, C.c_char_p, _I]),
     "pcf_autotune_batch": (_I, [_P, _I, _I, C.POINTER(McRequest), C.c_char_p, _I]),
     "pcf_tune_report": (_I, [_P, C.c_char_p, _I]),

@@ -90,6 +90,12 @@ class Context:
         _lib.check(_lib.load().pcf_ctx_set_test_lattice(self._h, int(withhold),
                                                          int(poll_limit)))
 
+    def set_test_strip_level(self, level: int) -> None:
+        """Test hook: the lattice strips take over at this level at the latest
+        (the kernel of large lattices runs the levels above it); 0 restores
+        normal operation."""
+        _lib.check(_lib.load().pcf_ctx_set_test_strip_level(self._h, int(level)))
+
     def autotune(self, mc: bool = True, lsm: bool = True, save: bool = False,
                  requests=None) -> dict:
         """Time candidate work shapes on this device and keep the fastest

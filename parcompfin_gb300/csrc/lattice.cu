@@ -526,7 +526,8 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
     }
     if (occ < 1) return set_error(PCF_EINVAL, "the lattice strip block does not fit on an SM");
     const int cap = occ * c->sm_count * kOwn * kStripWarps;
-    const int top = std::min(N, cap - 1);
+    int top = std::min(N, cap - 1);
+    if (c->test_strip_level) top = std::min(top, c->test_strip_level);  // test hook
     // The fewest warps per block that give each strip an SM of its own: up to
     // three warps of a block an FP64 instruction takes 64 cycles, four share
     // the pipe at 76 (measured).

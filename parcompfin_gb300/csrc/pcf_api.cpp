@@ -406,6 +406,17 @@ int pcf_ctx_set_test_lattice(pcf_ctx* ctx, int withhold, unsigned poll_limit) {
   });
 }
 
+int pcf_ctx_set_test_strip_level(pcf_ctx* ctx, int level) {
+  return pcf::abi_guard([&]() -> int {
+    int st;
+    pcf_ctx* c = resolve_ctx(ctx, &st);
+    if (!c) return st;
+    if (level < 0) return set_error(PCF_EINVAL, "level must be >= 0");
+    c->test_strip_level = level;
+    return PCF_OK;
+  });
+}
+
 int pcf_mc_eur(pcf_ctx* ctx, double S0, double E, double r, double sigma, double T, long long N,
                int payoff_fun, unsigned long long seed, int use_cv, pcf_mc_result* out) {
   return pcf::abi_guard([&]() -> int {

@@ -51,6 +51,7 @@ struct pcf_ctx {
   unsigned test_barrier_extra = 0;
   unsigned test_poll_limit = 0;
   int test_lattice = 0;  // test hook (pcf_ctx_set_test_lattice): the wait to starve
+  int test_strip_level = 0;  // test hook (pcf_ctx_set_test_strip_level): 0, or the strips' top
   long long launches = 0;
 };
 

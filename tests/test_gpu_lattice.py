@@ -138,3 +138,46 @@ def test_lattice_starved_waits_give_up_then_recover(orc, ctx, withhold, N, ameri
     finally:
         ctx.set_test_lattice(0)
     assert fn(*args, N, -1, ctx=ctx) == ref(*args, N, -1.0)
+
+
+@pytest.mark.parametrize("american", [True, False])
+@pytest.mark.parametrize("args", [(100, 110, .02, .75, 1.0, -1), (50, 60, .08, .3, 2.0, 1),
+                                  (1e-280, 2e-280, .05, .2, 1.0, -1)])  # last: IEEE division
+@pytest.mark.parametrize("above", [1, 127, 128, 129, 256, 257])
+def test_lattice_blocked_levels_bit_exact(orc, ctx, above, args, american):
+    """The levels above the strips, 128 a grid step, and the hand-over: one
+    level, partial and whole steps, an odd and an even number of them (the two
+    level arrays alternate), above 800 and 2500 levels of strips."""
+    import parcompfin_gb300 as pcf
+    fn = pcf.binom_vanilla_amer if american else pcf.binom_vanilla_eur
+    ref = orc.ref_binom_vanilla_amer if american else orc.ref_binom_vanilla_eur
+    try:
+        for top in (800, 2500):
+            ctx.set_test_strip_level(top)
+            N = top + above
+            before = ctx.launches
+            got = fn(*args[:5], N, args[5], ctx=ctx)
+            assert ctx.launches - before in (2, 4)  # blocked and strips, once or twice
+            assert got == ref(*args[:5], N, float(args[5])), (N, top, args, american)
+    finally:
+        ctx.set_test_strip_level(0)
+
+
+def test_lattice_blocked_barrier_gives_up_then_recovers(orc, ctx):
+    """The grid barrier of the levels above the strips, waiting for a block
+    more than there are, gives up; the next call is the reference's price."""
+    import parcompfin_gb300 as pcf
+    from parcompfin_gb300._lib import PCF_ETIMEOUT, PcfError
+    args = (*CASES[0], 2757, -1)
+    try:
+        ctx.set_test_strip_level(2500)
+        ctx.set_test_barrier(1, 2000)
+        with pytest.raises(PcfError, match="grid barrier") as e:
+            pcf.binom_vanilla_amer(*args, ctx=ctx)
+        assert e.value.status == PCF_ETIMEOUT
+        ctx.set_test_barrier(0)
+        assert pcf.binom_vanilla_amer(*args, ctx=ctx) == orc.ref_binom_vanilla_amer(
+            *args[:6], float(args[6]))
+    finally:
+        ctx.set_test_barrier(0)
+        ctx.set_test_strip_level(0)
