@@ -528,30 +528,40 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
     const int cap = occ * c->sm_count * kOwn * kStripWarps;
     int top = std::min(N, cap - 1);
     if (c->test_strip_level) top = std::min(top, c->test_strip_level);  // test hook
-    // The fewest warps per block that give each strip an SM of its own: up to
-    // three warps of a block an FP64 instruction takes 64 cycles, four share
-    // the pipe at 76 (measured).
-    int W = kStripWarps;
-    for (int k = 1; k < kStripWarps; ++k)
-      if ((long long)k * kOwn * c->sm_count >= (long long)top + 1) {
-        W = k;
-        break;
-      }
-    const bool help = american && W < kStripWarps;
-    const int strips = (top + kOwn * W) / (kOwn * W);
-
-    // Scratch: up | dn | rings | counters (barrier, err, taken) | out and, for
-    // the blocked levels, A | B.
     const size_t nodes = (size_t)N + 1;
-    auto a256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t o_up = 0, o_dn = o_up + 8 * nodes;
-    const size_t o_ring = a256(o_dn + 8 * nodes);
-    const size_t ring_bytes = sizeof(unsigned long long) * kRing * (size_t)strips;
-    const size_t o_cnt = a256(o_ring + ring_bytes);
-    const size_t cnt_bytes = 256 + a256(sizeof(unsigned) * (size_t)strips);
+    int W = 0, strips = 0;
+    size_t o_ring = 0, ring_bytes = 0, o_cnt = 0, cnt_bytes = 0, o_A = 0, total = 0;
+    auto lay_out = [&]() {
+      // The fewest warps per block that give each strip an SM of its own: up to
+      // three warps of a block an FP64 instruction takes 64 cycles, four share
+      // the pipe at 76 (measured).
+      W = kStripWarps;
+      for (int k = 1; k < kStripWarps; ++k)
+        if ((long long)k * kOwn * c->sm_count >= (long long)top + 1) {
+          W = k;
+          break;
+        }
+      strips = top ? (top + kOwn * W) / (kOwn * W) : 0;
+      // Scratch: up | dn | rings | counters (barrier, err, out, taken) and, for
+      // the blocked levels, A | B.
+      auto a256 = [](size_t x) { return (x + 255) & ~(size_t)255; };
+      o_ring = a256(16 * nodes);
+      ring_bytes = sizeof(unsigned long long) * kRing * (size_t)strips;
+      o_cnt = a256(o_ring + ring_bytes);
+      cnt_bytes = 256 + a256(sizeof(unsigned) * (size_t)strips);
+      o_A = o_cnt + cnt_bytes;
+      total = o_A + (top < N ? 16 * nodes : 0);
+    };
+    lay_out();
+    // Where the memory limit has no room for the rings, the blocked kernel runs
+    // every level: slower, and no more scratch than two level arrays.
+    if (!ctx_fits(c, total)) {
+      top = 0;
+      lay_out();
+    }
+    const bool help = american && W < kStripWarps;
+    const size_t o_up = 0, o_dn = 8 * nodes, o_B = o_A + 8 * nodes;
     const size_t o_out = o_cnt + 128;  // beside the error word: one copy brings both
-    const size_t o_A = o_cnt + cnt_bytes, o_B = a256(o_A + (top < N ? 8 * nodes : 0));
-    const size_t total = o_B + (top < N ? 8 * nodes : 0);
     st = ctx_ensure(c, total, 16 * nodes + 256);
     if (st) return st;
     char* dv = (char*)c->d_buf;
@@ -604,7 +614,7 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
     for (;;) {
       st = cuda_status(cudaMemsetAsync(dv + o_cnt, 0, cnt_bytes, c->stream),
                        "memset lattice counters");
-      if (!st)
+      if (!st && strips)
         st = cuda_status(cudaMemsetAsync(dv + o_ring, 0xff, ring_bytes, c->stream),
                          "memset lattice rings");
       if (st) return st;
@@ -625,13 +635,18 @@ extern "C" int pcf_binom_vanilla(pcf_ctx* ctx, double S0, double E, double r, do
         c->launches += 1;
         P.src = ((N - top + kLatSteps - 1) / kLatSteps) % 2 ? P.B : P.A;
       }
-      void* args[] = {&P};
-      st = cuda_status(cudaLaunchCooperativeKernel((void*)strip_kernel(american != 0, exact, help),
-                                                   dim3(strips), dim3(32 * (W + 1 + help)), args, 0,
-                                                   c->stream),
-                       "lattice strip launch");
+      if (strips) {
+        void* args[] = {&P};
+        st = cuda_status(
+            cudaLaunchCooperativeKernel((void*)strip_kernel(american != 0, exact, help),
+                                        dim3(strips), dim3(32 * (W + 1 + help)), args, 0, c->stream),
+            "lattice strip launch");
+        if (!st) c->launches += 1;
+      } else {
+        st = cuda_status(cudaMemcpyAsync(P.out, P.src, 8, cudaMemcpyDeviceToDevice, c->stream),
+                         "lattice root");
+      }
       if (st) return st;
-      c->launches += 1;
       st = cuda_status(cudaMemcpyAsync(h, dv + o_cnt, 256, cudaMemcpyDeviceToHost, c->stream),
                        "D2H lattice");
       if (!st) st = cuda_status(cudaStreamSynchronize(c->stream), "lattice kernel");

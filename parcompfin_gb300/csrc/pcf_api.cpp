@@ -48,12 +48,18 @@ void ctx_release_extras(pcf_ctx* c) {
   c->d_ticket = nullptr;
 }
 
+static size_t scratch_bytes(size_t need) { return std::max(align256(need), (size_t)1 << 20); }
+
+bool ctx_fits(const pcf_ctx* c, size_t dev_bytes) {
+  return dev_bytes <= c->d_cap || !c->budget_bytes || scratch_bytes(dev_bytes) <= c->budget_bytes;
+}
+
 int ctx_ensure(pcf_ctx* c, size_t dev_bytes, size_t host_bytes) {
   if (dev_bytes > c->d_cap) {
     if (c->d_buf) cudaFree(c->d_buf);
     c->d_buf = nullptr;
     c->d_cap = 0;
-    const size_t want = std::max(align256(dev_bytes), (size_t)1 << 20);
+    const size_t want = scratch_bytes(dev_bytes);
     if (c->budget_bytes && want > c->budget_bytes)
       return set_error(PCF_ENOMEM, "scratch of %zu bytes exceeds the context budget of %zu",
                        want, c->budget_bytes);

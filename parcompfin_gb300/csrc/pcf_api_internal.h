@@ -76,6 +76,8 @@ int abi_guard(Body&& body) noexcept {
 }
 int cuda_status(cudaError_t e, const char* what);
 int ctx_ensure(pcf_ctx* c, size_t dev_bytes, size_t host_bytes);
+// Whether the memory limit lets ctx_ensure have dev_bytes of device scratch.
+bool ctx_fits(const pcf_ctx* c, size_t dev_bytes);
 pcf_ctx* resolve_ctx(pcf_ctx* ctx, int* status);
 void ctx_release_extras(pcf_ctx* c);
 void serve_release(pcf_ctx* c);  // frees the serving slots (pcf_server.cpp)

@@ -181,3 +181,23 @@ def test_lattice_blocked_barrier_gives_up_then_recovers(orc, ctx):
     finally:
         ctx.set_test_barrier(0)
         ctx.set_test_strip_level(0)
+
+
+@pytest.mark.parametrize("american", [True, False])
+def test_lattice_under_a_memory_limit(orc, pcf_lib, american):
+    """The strips' rings (8 KB a strip) are scratch that the levels above them
+    do without: a limit that leaves no room for them is no refusal, and the
+    price is the same."""
+    import parcompfin_gb300 as pcf
+    fn = pcf.binom_vanilla_amer if american else pcf.binom_vanilla_eur
+    ref = orc.ref_binom_vanilla_amer if american else orc.ref_binom_vanilla_eur
+    for N in (3300, 20_000):
+        with pcf.Context(0) as c:
+            c.set_memory_limit(1 << 20)
+            for args in CASES[:2]:
+                assert fn(*args, N, -1, ctx=c) == ref(*args, N, -1.0), (N, args, american)
+            if N < 10_000:  # the IEEE division
+                args = (1e-280, 2e-280, .05, .2, 1.0, N)
+                assert fn(*args, -1, ctx=c) == ref(*args, -1.0)
+            with pytest.raises(pcf.PcfError, match="budget"):
+                fn(*CASES[0], 40_000, -1, ctx=c)
