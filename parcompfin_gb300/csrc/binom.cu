@@ -971,6 +971,12 @@ extern "C" int pcf_binom_embar_batch(pcf_ctx* ctx, int n, const pcf_binom_contra
     const size_t o_prep = a256(o_tick + sizeof(unsigned) * n);
     const size_t o_map = a256(o_prep + sizeof(BinomPrep) * n);
     const size_t total = a256(o_map + sizeof(int) * items);
+    if (n > 1 && !ctx_fits(c, total)) {
+      // The memory limit has no room for the whole batch (a contract takes some
+      // 500 bytes, most of them its BinomPrep): in two parts.
+      st = pcf_binom_embar_batch(c, n / 2, ks, mode, prices);
+      return st ? st : pcf_binom_embar_batch(c, n - n / 2, ks + n / 2, mode, prices + n / 2);
+    }
     st = ctx_ensure(c, total, h2d + sizeof(double) * n);
     if (st) return st;
     char* h = (char*)c->h_buf;

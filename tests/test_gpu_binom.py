@@ -269,3 +269,17 @@ def test_accurate_mode_away_from_even_odds(orc, ctx, r, sig, T, N, sign):
     for c, v in zip(cs, binom_embar_batch(cs, mode="accurate", ctx=ctx)):
         ref = _exact_binom(orc, *c)
         assert abs(v - ref) <= (8 + 2 * math.sqrt(N)) * 2**-52 * ref, (c, v, ref, rel(v, ref))
+
+
+@pytest.mark.parametrize("mode", ["reference", "accurate"])
+def test_batch_under_a_memory_limit(ctx, mode):
+    """A batch whose scratch exceeds the context's limit is priced in parts,
+    with the prices of the whole batch."""
+    from parcompfin_gb300 import Context, binom_embar_batch
+    rng = random.Random(11)
+    cs = [(100.0, rng.uniform(80, 120), rng.uniform(.01, .06), rng.uniform(.1, .5),
+           rng.uniform(.25, 2.0), rng.randint(1, 300), rng.choice([1, -1])) for _ in range(5001)]
+    want = binom_embar_batch(cs, mode=mode, ctx=ctx)
+    with Context(0) as c:
+        c.set_memory_limit(1 << 20)
+        assert binom_embar_batch(cs, mode=mode, ctx=c) == want
