@@ -1133,32 +1133,34 @@ __global__ void __launch_bounds__(kLsmCBlock, J > 2 ? 1 : 2)
 }
 
 // Groups of four pairs a thread of a 512-thread block holds for a slice of PB
-// pairs: the kernels' J.
+// pairs: the kernels' J, at most kMaxGroups. lsm_fits turns larger slices away.
+constexpr int kMaxGroups = 4;
+constexpr int kMaxSlice = 4 * kMaxGroups * kLsmBlock;  // pairs a block
 int lsm_groups(int PB) {
   const int k = (PB / 4 + kLsmBlock - 1) / kLsmBlock;
-  return k <= 1 ? 1 : k <= 2 ? 2 : 4;
+  return k <= 1 ? 1 : k <= 2 ? 2 : kMaxGroups;
 }
 static_assert(kLsmBlock == kLsmCBlock, "lsm_groups serves both");
 typedef void (*LsmKernel)(LsmParams);
 typedef void (*LsmClusterKernel)(const LsmParams*, int);
 LsmKernel lsm_kernel_for(int PB) {
   const int k = lsm_groups(PB);
-  return k == 1 ? lsm_kernel<1> : k == 2 ? lsm_kernel<2> : lsm_kernel<4>;
+  return k == 1 ? lsm_kernel<1> : k == 2 ? lsm_kernel<2> : lsm_kernel<kMaxGroups>;
 }
 LsmKernel lsm_hybrid_for(int PB) {
   const int k = lsm_groups(PB);
   return k == 1 ? lsm_coop_cluster_kernel<1> : k == 2 ? lsm_coop_cluster_kernel<2>
-                                                      : lsm_coop_cluster_kernel<4>;
+                                                      : lsm_coop_cluster_kernel<kMaxGroups>;
 }
 LsmClusterKernel lsm_cluster_for(int PB, bool t8) {
   const int k = lsm_groups(PB);
   if (t8)
     return k == 1   ? lsm_cluster_kernel<unsigned char, 1>
            : k == 2 ? lsm_cluster_kernel<unsigned char, 2>
-                    : lsm_cluster_kernel<unsigned char, 4>;
+                    : lsm_cluster_kernel<unsigned char, kMaxGroups>;
   return k == 1   ? lsm_cluster_kernel<unsigned short, 1>
          : k == 2 ? lsm_cluster_kernel<unsigned short, 2>
-                  : lsm_cluster_kernel<unsigned short, 4>;
+                  : lsm_cluster_kernel<unsigned short, kMaxGroups>;
 }
 
 // Dynamic shared memory of one block (the carve above).
@@ -1262,7 +1264,7 @@ const LsmLimits& lsm_limits(const pcf_ctx* c) {
     L.status = cuda_status(
         cudaDeviceGetAttribute(&v, cudaDevAttrReservedSharedMemoryPerBlock, c->device), "attr");
   L.reserved = (size_t)v;
-  for (int PB : {kLsmBlock * 4, kLsmBlock * 8, kLsmBlock * 16}) {
+  for (int PB : {kLsmBlock * 4, kLsmBlock * 8, kMaxSlice}) {
     auto setup = [&](auto kernel, size_t& most, bool cluster) {
       size_t stat = 0;
       if (!L.status) L.status = lsm_kernel_setup(kernel, L.per_block, &stat, cluster);
@@ -1301,6 +1303,7 @@ const LsmLimits& lsm_limits(const pcf_ctx* c) {
 
 bool lsm_fits(const LsmLimits& Lm, int PB, int M, size_t tau_bytes, size_t stat, int per_sm) {
   const size_t need = lsm_smem(PB, M, tau_bytes) + stat;
+  if (PB > kMaxSlice) return false;  // a thread holds no more than kMaxGroups groups
   return need <= Lm.per_block && (size_t)per_sm * (need + Lm.reserved) <= Lm.per_sm;
 }
 
@@ -1421,6 +1424,7 @@ int launch_coop(const LsmParams& P0, int G, int PB, size_t smem, int hcl, int Gh
 
 constexpr int kLsmPB[] = {512, 1024, 2048, 4096, 8192};
 constexpr int kNumPB = 5;
+static_assert(kLsmPB[kNumPB - 1] <= kMaxSlice, "the kernels hold kMaxSlice pairs a block");
 
 // Shape of a contract in a cluster launch: the smallest power-of-two cluster
 // that covers the contract with slices that let two CTAs share an SM (the

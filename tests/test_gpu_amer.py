@@ -360,3 +360,14 @@ def test_amer_batch_slices_match_fp64_twin(orc, ctx, N, M):
     assert s[5] == 0
     for k in (0, 2):
         assert abs(res.sums[k] - s[k]) <= 3e-4 * abs(s[k]), (k, res.sums[k], s[k])
+
+
+@pytest.mark.parametrize("pairs_per_block", [4096, 4100, 8160, 8192, 8196, 12_292])
+def test_amer_largest_slices(orc, ctx, pairs_per_block):
+    """Slices around the most that a block's threads hold (8192 pairs, beyond
+    which the sweep streams) and around the steps below it: every path is
+    regressed and decided, none is left out. Blocks: one an SM."""
+    res, a = audit(orc, ctx, 100, 100, .05, .3, 1.0, 2 * 152 * pairs_per_block, 3, -1, False, 5)
+    assert a["r1_tau_mismatch"] == 0 and a["r1_mode_mismatch"] == 0, a
+    assert a["sums_rel_err"] < 1e-6 and a["regression_dates"] == 2, a
+    assert a["price_rel_err_same_policy"] < 1e-5, a
