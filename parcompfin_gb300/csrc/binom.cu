@@ -93,7 +93,7 @@ struct BinomTables {
 };
 
 struct BinomContract {
-  double S0, E, u, d, lp, lq, logu, logd;
+  double S0, E, u, d, lp, lq;
   double p, q;   // accurate mode
   double stirl_n, twopi_n;  // accurate mode: stirlerr(N), 2 pi / N
   int N, pf, i_lo, i_hi;  // pair indices i_lo..i_hi (inclusive)
@@ -121,7 +121,7 @@ struct BinomPrep {
 struct BinomLaunch {
   const BinomContract* cs;
   const int* item_start;
-  int ncontracts, total_items;
+  int ncontracts;
   double* partial;
   unsigned* tickets;
   double* out;
@@ -905,8 +905,6 @@ int setup_contract(const pcf_binom_contract& k, int idx, BinomContract& C) {
   C.q = q;
   C.lp = log(p);
   C.lq = log(q);
-  C.logu = log(u);
-  C.logd = log(d);
   C.twopi_n = 2 * 3.14159265358979323846 / N;
   if (N <= 15) {
     double small[16];
@@ -917,7 +915,7 @@ int setup_contract(const pcf_binom_contract& k, int idx, BinomContract& C) {
   }
   // The reference's pow(u, i), pow(d, N - i) and S0 pow(u, i) stay inside the
   // FP64 range for every i <= N.
-  const double span = std::max(fabs(C.logu), fabs(C.logd)) * N + fabs(log(k.S0));
+  const double span = std::max(fabs(log(u)), fabs(log(d))) * N + fabs(log(k.S0));
   C.wide = span < 690.0 ? 0 : 1;
   C.N = N;
   C.pf = pf;
@@ -990,7 +988,6 @@ extern "C" int pcf_binom_embar_batch(pcf_ctx* ctx, int n, const pcf_binom_contra
     L.cs = (const BinomContract*)(d + o_cs);
     L.item_start = (const int*)(d + o_start);
     L.ncontracts = n;
-    L.total_items = items;
     L.partial = (double*)(d + o_part);
     L.tickets = (unsigned*)(d + o_tick);
     L.out = out;
