@@ -25,15 +25,17 @@
 // mode 1 (accurate): log C(N,k) p^k q^{N-k} by Loader's saddle-point
 //   formula (C. Loader, "Fast and Accurate Computation of Binomial
 //   Probabilities", 2000: Stirling-series remainders plus bd0 deviance
-//   terms), accurate to ~1e-15 relative per term.
+//   terms), accurate to some 1e-15 + |k - N p| 2^-53 relative per term (N p
+//   is rounded): prices of N = 2001 .. 50,001 with p = 0.36 .. 0.64 are within
+//   4e-14 of 60-digit sums.
 //
 // Two kernels a batch (GB300, 1024 contracts of N = 1e3 .. 2e5, 2.6 million
 // terms: 3.67 ms before, 0.28 ms now; accurate mode 4.6 -> 0.5 ms):
 //   binom_prep_kernel  walks the additions of the contract's accumulator once
 //            (they are the same for every term up to where it subtracts; a walk
 //            per term was 85 % of the integer work) and takes the logarithms of
-//            u, d and S0 to 96 bits after the point. Bound by the latency of
-//            its chain of loads, 48 us.
+//            u, d and S0 (in the accurate mode p and 1 - p too) to 96 bits
+//            after the point. Bound by the latency of its chain of loads, 48 us.
 //   binom_kernel       one thread a pair of terms. The FP64 pipe is the scarce
 //            unit of GB300 (19 cycles a warp instruction and SM against 0.25 for
 //            the other pipes), so only the reference's own additions and
@@ -454,7 +456,10 @@ __global__ void __launch_bounds__(kBinomBlock) binom_wide_kernel(BinomLaunch L) 
 // high product on the integer pipe takes 4.8. pow and exp in FP64 were about
 // 650 of a term's 700 FP64 operations and the kernel's bound, so both are
 // evaluated as powers of two in fixed point, to 2^-57 relative, and only the
-// reference's own additions and products remain in FP64.
+// reference's own additions and products remain in FP64. (A power's exponent has
+// 64 bits after the point; an exponential's, |b| log2(e), has 62 - e for |b| in
+// [2^e, 2^(e+1)): 2^-57 relative up to |b| = 64, 2^-53 at the smallest weights
+// that are not 0, |b| = 690.)
 
 // 2^-f for a fraction f in units of 2^-64, in units of 2^-63. With f = j/256 + r
 // and x = r ln 2 < 2^-8.5: 2^-f = T[j] (1 - c), c = 1 - e^-x = x (1 - h),

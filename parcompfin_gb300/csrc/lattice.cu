@@ -27,9 +27,11 @@
 // limits the proof to s >= 2^-960; nodes below that differ by at most the last
 // bit of a value that weighs below 2^-260 of any price of 2^-700 or more, and
 // a smaller or non-finite price is computed again with the IEEE division
-// (kExact), as is every lattice whose R, p or q is out of the ordinary range.
+// (EXACT), as is every lattice whose R, p or q is out of the ordinary range or
+// whose nodes may be infinite or not a number (lat_leaves_range).
 //
-// Two kernels:
+// Two kernels (where a memory limit leaves no room for the strips' rings, the
+// blocked one alone):
 //   strips   columns i are cut into strips of 24 W (W = 1..4 warps, 24 columns
 //            each). A level needs only v[i] and v[i+1], so values flow from
 //            right to left and a node stays in its thread's register for the

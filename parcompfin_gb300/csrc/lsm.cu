@@ -1197,7 +1197,7 @@ void lsm_fill(LsmParams& P, double S0, double E, double r, double sigma, double 
   P.seed_lo = (uint32_t)seed;
   P.seed_hi = (uint32_t)(seed >> 32);
   P.stream = stream;
-  P.wait_limit = 1u << 22;       // ~32 ns sleep + an L2 round trip per poll: seconds
+  P.wait_limit = 1u << 22;       // an L2 round trip per poll: seconds
   P.copy_wait_limit = 1u << 20;  // try_wait polls: far beyond a microsecond-scale wait
 }
 
